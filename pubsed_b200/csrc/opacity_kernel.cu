@@ -32,6 +32,7 @@
 // outputs are passed offset to the chunk, and every scratch array
 // (index * nzones + zone) is sized for one chunk, so a 128^3-zone grid with
 // thousands of bins builds its tables through a bounded working set.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <mutex>
@@ -245,9 +246,9 @@ struct LevView {
 // atom's number density, n_l n_atom, and their reciprocals (or the ion
 // populations for fuzz lines) are staged in shared memory level-major, ZT
 // zones contiguous; the ratio n_u g_l / (n_l g_u) is formed from them (the
-// atom density cancels).  A warp takes one bin at a time (warp w the bins
-// order[w], order[w + 8], ..., `order` listing the bins by decreasing line
-// count): its lanes are ZT zones x 32/ZT line slots, slot s summing the
+// atom density cancels).  A warp takes one bin at a time (the warps of the
+// gridDim.y CTAs of a tile deal the bins of `order`, which lists them by
+// decreasing line count, among themselves): its lanes are ZT zones x 32/ZT line slots, slot s summing the
 // bin's lines s, s + 32/ZT, ... (sorted by bin, atom), and the slots of a
 // zone are then added in FP64 in a fixed butterfly order, so the sums are
 // the same from run to run.  The FP64 form sums in FP64; the mixed form
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(32 * LINE_SUM_WARPS) line_sum_kernel(const Opa
   // line loop is unrolled by two (Type Ia 6.9 -> 5.4 ms before the staging).
   constexpr int LS = 32 / ZT;
   static_assert(32 % LS == 0, "a slot keeps its lines across the 32-record chunks");
-  const int lane = tid & 31, warp = tid >> 5, nwarps = bd >> 5;
+  const int lane = tid & 31, warp = tid >> 5, nwarps = (bd >> 5) * gridDim.y;
   const int zi = lane % ZT, slot = lane / ZT;
   using CRec = typename std::conditional<MIXED, typename std::conditional<FUZZ, float4, float2>::type, double2>::type;
   __shared__ int4 s_ix[LINE_SUM_WARPS][32];
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(32 * LINE_SUM_WARPS) line_sum_kernel(const Opa
   } else {
     cr_g = FUZZ ? A.fz_c : A.ln_c;
   }
-  for (int jj = warp; jj < nn; jj += nwarps) {
+  for (int jj = warp * gridDim.y + blockIdx.y; jj < nn; jj += nwarps) {
     const int j = __ldg(order + jj);
     double acc = 0, acce = 0;
     float ks = 0.f, kc = 0.f, kse = 0.f, kce = 0.f;  // the mixed form's FP32 Kahan sums
@@ -737,8 +738,17 @@ __global__ void __launch_bounds__(256) zone_opacity_kernel(const OpacityArgs A)
 constexpr int LINE_TILE_MIXED = 8;
 constexpr int LINE_TILE_FP64 = 4;
 
+// CTAs per tile: with few zones (a 1D model has 256, 32 tiles of 8) a CTA per
+// tile left most SMs without work, so the bins of a tile are dealt over as
+// many CTAs as bring the grid to LINE_SUM_CTAS_PER_SM per SM (the 2048 threads
+// an SM holds), but at least one bin per warp.  A bin is summed by one warp in
+// either case: the sums do not depend on the split.  On B200, FP32: 256 zones x
+// 4096 bins x 5e5 lines 3.18 ms -> 344 us, 128 x 2048 x 1e5 725 -> 47 us, 97 x
+// 1500 x 3e4 293 -> 21 us; 18 494 zones (2312 tiles, unsplit as before) 2.03 ms.
+constexpr int LINE_SUM_CTAS_PER_SM = 8;
+
 template <bool MIXED, bool FUZZ>
-int launch_line_sums(const OpacityArgs& a, double* S, double* Se, cudaStream_t s)
+int launch_line_sums(const OpacityArgs& a, double* S, double* Se, int num_sms, cudaStream_t s)
 {
   constexpr int ZT = MIXED ? LINE_TILE_MIXED : LINE_TILE_FP64;
   const size_t vs = MIXED ? sizeof(float) : sizeof(double);
@@ -746,7 +756,11 @@ int launch_line_sums(const OpacityArgs& a, double* S, double* Se, cudaStream_t s
   const size_t smem = vs * ((size_t)a.natoms * ZT + a.natoms + ZT + 2 * np * ZT);
   auto k = line_sum_kernel<MIXED, FUZZ, ZT>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
-  k<<<(a.nzones + ZT - 1) / ZT, 256, smem, s>>>(a, S, Se);
+  const int tiles = (a.nzones + ZT - 1) / ZT;
+  const int bin_groups = (a.n_nu + LINE_SUM_WARPS - 1) / LINE_SUM_WARPS;
+  const int want = (num_sms * LINE_SUM_CTAS_PER_SM + tiles - 1) / tiles;
+  const dim3 grid((unsigned)tiles, (unsigned)std::min(std::min(want, bin_groups), 65535));
+  k<<<grid, 32 * LINE_SUM_WARPS, smem, s>>>(a, S, Se);
   return 1;
 }
 
@@ -768,7 +782,6 @@ size_t line_sum_smem_bytes(int precision, int natoms, int n_pop)
 
 int launch_opacity(const OpacityArgs& a, int num_sms, cudaStream_t s)
 {
-  (void)num_sms;
   const int nz = a.nzones;
   int n = 0;
   zone_state_kernel<<<(nz + 127) / 128, 128, 0, s>>>(a, a.boltz);
@@ -776,14 +789,14 @@ int launch_opacity(const OpacityArgs& a, int num_sms, cudaStream_t s)
   const bool micro = a.natoms > 0;
   int r = 0;
   if (micro && a.use_line)
-    r = a.precision ? launch_line_sums<true, false>(a, a.abs64, a.epsl64, s)
-                    : launch_line_sums<false, false>(a, a.abs64, a.epsl64, s);
+    r = a.precision ? launch_line_sums<true, false>(a, a.abs64, a.epsl64, num_sms, s)
+                    : launch_line_sums<false, false>(a, a.abs64, a.epsl64, num_sms, s);
   if (r < 0) return -1;
   n += r;
   r = 0;
   if (micro && a.use_fuzz)
-    r = a.precision ? launch_line_sums<true, true>(a, a.scat64, a.epsf64, s)
-                    : launch_line_sums<false, true>(a, a.scat64, a.epsf64, s);
+    r = a.precision ? launch_line_sums<true, true>(a, a.scat64, a.epsf64, num_sms, s)
+                    : launch_line_sums<false, true>(a, a.scat64, a.epsf64, num_sms, s);
   if (r < 0) return -1;
   n += r;
   const size_t smem = opacity_smem_bytes(a);

@@ -1,0 +1,45 @@
+"""The opacity build against the oracle at the sizes where its split over the
+chip can go wrong: fewer bins than the warps of a CTA, bins that are no
+multiple of it, one zone, a zone more than a tile, many zones with few bins;
+both forms, with the tolerances of test_gpu_opacity.py."""
+import numpy as np
+import pytest
+
+from pubsed_b200 import abi, workloads
+import oracle_lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _maxrel(a, b):
+    s = np.abs(b)
+    s = np.where(s == 0, 1e-300, s)
+    return float(np.max(np.abs(a - b) / s))
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("n_zones,n_bins,n_lines", [(1, 300, 4000), (9, 7, 3000), (33, 65, 20000), (700, 20, 500),
+                                                    (5, 2049, 8000)])
+def test_opacity_shapes_match_oracle(sed_lib, precision, n_zones, n_bins, n_lines):
+    w = workloads.type_ia(n_packets=10, n_zones=n_zones, n_lines=n_lines, n_bins=n_bins, bound_free=1,
+                          n_levels_per_ion=7) if n_zones > 1 else _one_zone(n_bins, n_lines)
+    o = oracle_lib.Engine(oracle_lib.oracle_lib(), "oracle_", w)
+    g = oracle_lib.Engine(sed_lib, "sed_", w, precision=precision)
+    for e in (o, g):
+        e.set_opacity(1.0)
+    Oo, Og = o.opacity(), g.opacity()
+    tol = 1e-12 if precision == abi.PREC_FP64 else 1e-5
+    assert _maxrel(Og["n_elec"], Oo["n_elec"]) <= 1e-12
+    for k in ("abs", "scat", "planck_mean", "rosseland_mean", "L_thermal"):
+        assert _maxrel(Og[k], Oo[k]) <= tol, k
+    assert np.max(np.abs(Og["emis_cdf"] - Oo["emis_cdf"])) <= tol  # CDF entries lie in [0, 1]
+    o.close()
+    g.close()
+
+
+def _one_zone(n_bins, n_lines):
+    w = workloads.type_ia(n_packets=10, n_zones=2, n_lines=n_lines, n_bins=n_bins, bound_free=1, n_levels_per_ion=7)
+    z = w.zones
+    for k in ("rho", "T", "X", "vol", "r_out", "v"):
+        setattr(z, k, getattr(z, k)[1:])
+    return w
