@@ -1,7 +1,9 @@
 // opacity_kernel.cu -- per-zone opacity/emissivity build on the device
 // (transport::set_opacity, src/transport/transport_opacity.cpp:21-260).
 //
-//   zone_state_kernel   one thread per zone: temperature clamp, mass
+//   zone_state_warp_kernel
+//                       one warp per zone (zone_state_kernel, one thread,
+//                       for very long level lists): temperature clamp, mass
 //                       fractions, then the LTE electron-density solve
 //                       (GasState::solve_state / ne_brent_method,
 //                       src/opacity/GasState.cpp:208-337) with
@@ -94,15 +96,16 @@ __device__ double charge_conservation(const OpacityArgs& A, int z, double ne, do
   return f - ne;
 }
 
-// GasState::ne_brent_method (GasState.cpp:270-337); *last = last point evaluated
-__device__ double ne_brent(const OpacityArgs& A, int z, double T, double dens, const double* boltz_e, double x1,
-                           double x2, double tol, double* last, int* err)
+// GasState::ne_brent_method (GasState.cpp:270-337) on f(ne), the charge
+// conservation of one zone; *last = last point evaluated
+template <class F>
+__device__ double ne_brent(F& f, double x1, double x2, double tol, double* last, int* err)
 {
   const int ITMAX = 100;
   const double EPS = 3.0e-8;
   double a = x1, b = x2, c = x2, d = 0, e = 0, min1, min2;
-  double fa = charge_conservation(A, z, a, T, dens, boltz_e, 0);
-  double fb = charge_conservation(A, z, b, T, dens, boltz_e, 0);
+  double fa = f(a);
+  double fb = f(b);
   *last = b;
   double fc, p, q, r, s, tol1, xm;
   if ((fa > 0.0 && fb > 0.0) || (fa < 0.0 && fb < 0.0)) *err = 1;
@@ -132,33 +135,48 @@ __device__ double ne_brent(const OpacityArgs& A, int z, double T, double dens, c
     a = b;
     fa = fb;
     b += (fabs(d) > tol1) ? d : (xm >= 0.0 ? fabs(tol1) : -fabs(tol1));
-    fb = charge_conservation(A, z, b, T, dens, boltz_e, 0);
+    fb = f(b);
     *last = b;
   }
   *err = 2;
   return 0.0;
 }
 
-__global__ void zone_state_kernel(const OpacityArgs A, double* boltz_e)
+// a zone's clamped temperature, mass fractions (GasState::set_mass_fractions,
+// GasState.cpp:137-156) and mean ion mass number
+__device__ __forceinline__ double zone_temperature(const OpacityArgs& A, int z)
 {
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nz = A.nzones;
-  if (z >= nz) return;
   double T = A.T[z];
   if (T < A.temp_min) T = A.temp_min;
   if (T > A.temp_max) T = A.temp_max;
-  A.temp_c[z] = T;
-  const double dens = A.rho[z];
-  // GasState::set_mass_fractions (GasState.cpp:137-156)
+  return T;
+}
+
+__device__ __forceinline__ double zone_mass_fractions(const OpacityArgs& A, int z, bool write)
+{
   double norm = 0.0;
   for (int a = 0; a < A.nelem; ++a) norm += A.X[(size_t)z * A.nelem + a];
   double inv = 0.;
   for (int a = 0; a < A.nelem; ++a) {
     const double mf = A.X[(size_t)z * A.nelem + a] / norm;
-    A.mass_frac[(size_t)a * nz + z] = mf;
+    if (write) A.mass_frac[(size_t)a * A.nzones + z] = mf;
     inv += mf / A.eA[a];
   }
-  const double mu_I = 1. / inv;
+  return 1. / inv;
+}
+
+// One thread per zone: the form for level lists too long for the shared
+// memory of zone_state_warp_kernel, and for FP64 chunks of very many zones
+// (launch_zone_state).
+__global__ void zone_state_kernel(const OpacityArgs A, double* boltz_e)
+{
+  const int z = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nz = A.nzones;
+  if (z >= nz) return;
+  const double T = zone_temperature(A, z);
+  A.temp_c[z] = T;
+  const double dens = A.rho[z];
+  const double mu_I = zone_mass_fractions(A, z, true);
   A.solve_err[z] = 0;
   if (A.grey[z] != 0 || A.natoms == 0) { A.n_elec[z] = 0; return; }
   for (int a = 0; a < A.natoms; ++a)
@@ -179,10 +197,208 @@ __global__ void zone_state_kernel(const OpacityArgs A, double* boltz_e)
   const double min_ne = 1e-10 * dens / (mu_I * MASS_P);
   double last = 0;
   int err = 0;
-  const double ne = ne_brent(A, z, T, dens, boltz_e, min_ne, max_ne, 1e-3, &last, &err);
+  auto f = [&](double ne) { return charge_conservation(A, z, ne, T, dens, boltz_e, 0); };
+  const double ne = ne_brent(f, min_ne, max_ne, 1e-3, &last, &err);
   charge_conservation(A, z, last, T, dens, boltz_e, 1);  // populations of the last evaluation
   A.n_elec[z] = ne;
   A.solve_err[z] = err;
+}
+
+// One warp per zone, ZONE_WARPS neighbouring zones per CTA, the zone's LTE
+// state in shared memory.  What bounds the solve is a chain: some 30 Brent
+// evaluations, each a pass over the ion stages and the levels.  One thread per
+// zone walked that chain alone, its state in global scratch: 2.2 ms for any
+// 1D model (one or two CTAs at work).  Here the lanes share the levels, lane a
+// the stages and the sum of atom a.
+//
+// The per-level terms, the stage recursion of each atom and every sum are the
+// reference's, in its order, so the FP64 form's populations are the same to
+// the bit.  With FP32 tables (FAST) an evaluation takes the mean charge of an
+// atom from its stage fractions, sum_i i f_i, instead of summing v_l i over
+// the levels: the level populations of a stage add up to f_i by construction,
+// so the two differ by rounding, and by the floor of 1e-30 per level, which
+// is below 1e-15 of any n_e inside the solver's bracket (n_e >= 1e-10 of the
+// ions).  An evaluation is then a dozen operations per stage instead of two
+// dozen per level.  On B200, against one thread per zone: 256 zones x 606
+// levels 2.2 ms -> 63 us (FP64 132 us), 18 494 zones 3.8 ms -> 344 us, 64^3
+// zones x 906 levels 18.7 -> 6.0 ms.
+constexpr int ZONE_WARPS = 4;  // 4 zones x 8 B: the CTA's level-major results fill whole 32 B sectors
+
+// doubles of shared memory per zone
+__host__ __device__ inline size_t zone_state_doubles(bool fast, int na, int ni, int nl)
+{
+  return (size_t)(fast ? 1 : 2) * nl + 3 * (size_t)ni + 2 * (size_t)na;
+}
+
+// stage fractions of atom a at electron density ne (AtomicSpecies::solve_lte,
+// AtomicSpecies_state.cpp:70-90): c[i] = exp(-chi/kT) part_i / part_(i-1)
+__device__ __forceinline__ void stage_fractions(double* fr, const double* c, int ni, double ne, double fac)
+{
+  fr[0] = 1.;
+  for (int i = 1; i < ni; ++i) {
+    double fi = c[i] * fac * fr[i - 1];
+    if (ne < 1e-50) fi = 0;
+    fr[i] = fi;
+    double norm = 0;
+    for (int j = 0; j <= i; j++) norm += fr[j];
+    for (int j = 0; j <= i; j++) fr[j] = fr[j] / norm;
+  }
+}
+
+template <bool FAST>
+__global__ void __launch_bounds__(32 * ZONE_WARPS) zone_state_warp_kernel(const OpacityArgs A)
+{
+  extern __shared__ double zsm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nz = A.nzones, na = A.natoms, nI = A.n_ions_total, nL = A.n_lev_total;
+  const int z0 = blockIdx.x * ZONE_WARPS, z = z0 + warp;
+  const size_t per = zone_state_doubles(FAST, na, nI, nL);
+  double* lev = zsm + warp * per;           // [nL] Boltzmann factors, then the populations (FAST); else the
+  double* eb = FAST ? lev : lev + nL;       // terms of the sums, then the populations, beside the factors
+  double* part = eb + nL;                   // [nI] partition functions
+  double* frac = part + nI;                 // [nI] stage fractions
+  double* coef = frac + nI;                 // [nI] exp(-chi/kT) part_i / part_(i-1)
+  double* nd = coef + nI;                   // [na] atom densities
+  double* net = nd + na;                    // [na] mean charges
+  bool micro = false;
+  if (z < nz) {
+    const double T = zone_temperature(A, z);
+    const double dens = A.rho[z];
+    const double mu_I = zone_mass_fractions(A, z, lane == 0);
+    micro = !(A.grey[z] != 0 || na == 0);
+    if (lane == 0) {
+      A.temp_c[z] = T;
+      A.solve_err[z] = 0;
+      if (!micro) A.n_elec[z] = 0;
+    }
+    if (micro) {
+      __syncwarp();  // lane 0's mass fractions
+      for (int a = lane; a < na; a += 32) nd[a] = dens * A.mass_frac[(size_t)a * nz + z] / (A.eA[a] * MASS_P);
+      for (int l = lane; l < nL; l += 32) eb[l] = exp(-A.lev_E[l] / K_EV / T);
+      __syncwarp();
+      for (int i = lane; i < nI; i += 32) {  // a stage's levels in order, a lane per stage
+        int a = 0;
+        while (A.ion_off[a + 1] <= i) ++a;
+        const int ion = i - A.ion_off[a], l1 = A.lev_off[a + 1];
+        double sum = 0;
+        for (int l = A.lev_off[a]; l < l1; ++l)
+          if (A.lev_ion[l] == ion) sum += A.lev_g[l] * eb[l];
+        part[i] = sum;
+      }
+      __syncwarp();
+      for (int i = lane; i < nI; i += 32) {
+        int a = 0;
+        while (A.ion_off[a + 1] <= i) ++a;
+        if (i > A.ion_off[a]) coef[i] = exp(-1.0 * A.ion_chi[i - 1] / K_EV / T) * (part[i] / part[i - 1]);
+      }
+      __syncwarp();
+      const double lt = H_PLANCK * H_PLANCK / (2.0 * PI * MASS_E * K_BOLTZ * T);
+      const double lt15 = pow(lt, 1.5);
+      // level populations at the current stage fractions, times the charge for the sum over levels
+      auto levels = [&](bool charge) {
+        for (int a = 0; a < na; ++a) {
+          const int i0 = A.ion_off[a], l1 = A.lev_off[a + 1];
+          for (int l = A.lev_off[a] + lane; l < l1; l += 32) {
+            const int ion = A.lev_ion[l];
+            double v = frac[i0 + ion] * A.lev_g[l] * eb[l] / part[i0 + ion];
+            if (v < 1e-30) v = 1e-30;
+            lev[l] = charge ? v * ion : v;
+          }
+        }
+        __syncwarp();
+      };
+      auto stages = [&](double ne) {
+        const double fac = 2 / ne / lt15;
+        for (int a = lane; a < na; a += 32) {
+          const int i0 = A.ion_off[a];
+          stage_fractions(frac + i0, coef + i0, A.ion_off[a + 1] - i0, ne, fac);
+        }
+        __syncwarp();
+      };
+      auto f = [&](double ne) {
+        if constexpr (FAST) {
+          const double fac = 2 / ne / lt15;
+          for (int a = lane; a < na; a += 32) {
+            const int i0 = A.ion_off[a], ni = A.ion_off[a + 1] - i0;
+            double u = 1., sum = 1., q = 0.;  // stage i to stage 0, their sum, the charge
+            for (int i = 1; i < ni; ++i) {
+              u = (ne < 1e-50) ? 0. : coef[i0 + i] * fac * u;
+              sum += u;
+              q += i * u;
+              if (sum > 1e100) { const double r = 1. / sum; u *= r; q *= r; sum = 1.; }
+            }
+            net[a] = q / sum;
+          }
+        } else {
+          stages(ne);
+          levels(true);
+          for (int a = lane; a < na; a += 32) {
+            double x = 0;
+            const int l1 = A.lev_off[a + 1];
+            for (int l = A.lev_off[a]; l < l1; ++l) x += lev[l];
+            net[a] = x;
+          }
+        }
+        __syncwarp();
+        double s = 0;
+        for (int a = 0; a < na; ++a) s += nd[a] * net[a];
+        __syncwarp();
+        return s - ne;
+      };
+      const double max_ne = 100 * dens / (mu_I * MASS_P);
+      const double min_ne = 1e-10 * dens / (mu_I * MASS_P);
+      double last = 0;
+      int err = 0;
+      const double ne = ne_brent(f, min_ne, max_ne, 1e-3, &last, &err);
+      stages(last);  // populations of the last evaluation
+      levels(false);
+      if (lane == 0) {
+        A.n_elec[z] = ne;
+        A.solve_err[z] = err;
+      }
+    }
+  }
+  // the CTA's results, the zones of a level next to each other
+  __shared__ int s_micro[ZONE_WARPS];
+  if (lane == 0) s_micro[warp] = micro;
+  __syncthreads();
+  auto put = [&](double* out, size_t off, int n) {
+    for (int i = threadIdx.x; i < n * ZONE_WARPS; i += 32 * ZONE_WARPS) {
+      const int q = i % ZONE_WARPS, k = i / ZONE_WARPS;
+      if (s_micro[q]) out[(size_t)k * nz + z0 + q] = zsm[q * per + off + k];
+    }
+  };
+  const size_t o = (FAST ? 1 : 2) * (size_t)nL;
+  put(A.lev_n, 0, nL);
+  put(A.ion_part, o, nI);
+  put(A.ion_frac, o + nI, nI);
+  put(A.n_dens, o + 3 * (size_t)nI, na);
+}
+
+// Shared memory a CTA of zone_state_warp_kernel may take: level lists beyond
+// it (about 3000 levels in FP64, 6000 with FP32 tables) take one thread per
+// zone.
+constexpr size_t ZONE_STATE_SMEM = 200 * 1024;
+// FP64 chunks of more zones than this take one thread per zone: with the chip
+// full of threads either way, the summing lanes' idle neighbours cost the warp
+// form more than the shared state saves it (906 levels: 64 000 zones 5.55
+// against 5.91 ms, 262 144 zones 22.2 against 18.2 ms).
+constexpr int ZONE_STATE_FP64_WARP_ZONES = 65536;
+
+int launch_zone_state(const OpacityArgs& a, cudaStream_t s)
+{
+  const bool fast = a.precision != 0;
+  const size_t smem = ZONE_WARPS * sizeof(double) * zone_state_doubles(fast, a.natoms, a.n_ions_total, a.n_lev_total);
+  if (smem > ZONE_STATE_SMEM || (!fast && a.nzones > ZONE_STATE_FP64_WARP_ZONES)) {
+    zone_state_kernel<<<(a.nzones + 127) / 128, 128, 0, s>>>(a, a.boltz);
+    return 1;
+  }
+  auto k = fast ? zone_state_warp_kernel<true> : zone_state_warp_kernel<false>;
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return -1;
+  k<<<(a.nzones + ZONE_WARPS - 1) / ZONE_WARPS, 32 * ZONE_WARPS, smem, s>>>(a);
+  return 1;
 }
 
 // ------------------------------------------------------------ per zone
@@ -784,7 +1000,7 @@ int launch_opacity(const OpacityArgs& a, int num_sms, cudaStream_t s)
 {
   const int nz = a.nzones;
   int n = 0;
-  zone_state_kernel<<<(nz + 127) / 128, 128, 0, s>>>(a, a.boltz);
+  if (launch_zone_state(a, s) < 0) return -1;
   ++n;
   const bool micro = a.natoms > 0;
   int r = 0;
@@ -906,6 +1122,6 @@ extern "C" int sed_lte_electron_density_noalloc(int32_t n_zones, const double* r
   // the array keeps the previous call's contents; only the grey-opacity
   // column must start at zero (every other entry is written before it is read)
   if (cudaMemsetAsync(grey, 0, nz * sizeof(double), s) != cudaSuccess) return SED_ERR_CUDA;
-  zone_state_kernel<<<(unsigned)((nz + 127) / 128), 128, 0, s>>>(A, A.boltz);
+  if (launch_zone_state(A, s) < 0) return SED_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SED_OK : SED_ERR_CUDA;
 }

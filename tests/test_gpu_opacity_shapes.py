@@ -43,3 +43,38 @@ def _one_zone(n_bins, n_lines):
     for k in ("rho", "T", "X", "vol", "r_out", "v"):
         setattr(z, k, getattr(z, k)[1:])
     return w
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("n_levels", [100, 200, 250])
+def test_long_level_lists_match_oracle(sed_lib, precision, n_levels):
+    """Level lists around the shared-memory limit of the warp-per-zone LTE
+    solve (3006, 6006 and 7506 levels): the last takes one thread per zone in
+    both forms, the second in FP64."""
+    w = workloads.type_ia(n_packets=10, n_zones=6, n_lines=500, n_bins=40, n_levels_per_ion=n_levels)
+    o = oracle_lib.Engine(oracle_lib.oracle_lib(), "oracle_", w)
+    g = oracle_lib.Engine(sed_lib, "sed_", w, precision=precision)
+    for e in (o, g):
+        e.set_opacity(1.0)
+    Oo, Og = o.opacity(), g.opacity()
+    assert _maxrel(Og["n_elec"], Oo["n_elec"]) <= 1e-12
+    for k in ("abs", "scat"):
+        assert _maxrel(Og[k], Oo[k]) <= (1e-12 if precision == abi.PREC_FP64 else 1e-5), k
+    o.close()
+    g.close()
+
+
+def test_fp64_lte_solve_is_the_same_in_both_forms(sed_lib, monkeypatch):
+    """68 921 cells solved in one chunk (a thread per zone) and in small chunks
+    (a warp per zone): the electron densities and tables are equal to the bit."""
+    w = workloads.cart3d(n_packets=10, n_cells=41, n_lines=50, n_bins=4, n_levels_per_ion=5)
+    out = []
+    for scratch in (None, str(32 << 20)):
+        if scratch:
+            monkeypatch.setenv("SEDONA_GPU_OPACITY_SCRATCH_BYTES", scratch)
+        g = oracle_lib.Engine(sed_lib, "sed_", w, precision=abi.PREC_FP64)
+        g.set_opacity(1.0)
+        out.append(g.opacity())
+        g.close()
+    for k in ("n_elec", "abs", "scat", "emis_cdf"):
+        assert np.array_equal(out[0][k], out[1][k]), k
