@@ -232,6 +232,9 @@ int sed_ctx_create(const sed_transport_params* p, int device, sed_ctx** out)
   CK(upload(c, c->d_sn, c->sn.x.data(), c->sn.x.size()));
   CK(upload(c, c->d_sm, c->sm.x.data(), c->sm.x.size()));
   CK(upload(c, c->d_sp, c->sp.x.data(), c->sp.x.size()));
+  CK(c->d_bin_tab.resize((size_t)BIN_TAB * c->nu.n()));
+  launch_bin_table(dev_loc(c->nu, c->d_nu), c->d_bin_tab.p, c->stream);
+  CK(cudaGetLastError());
   const std::vector<double> cdf = core_emission_cdf(c->nu, p->core_temperature);
   CK(upload(c, c->d_core_cdf, cdf.data(), cdf.size()));
   c->nspec = (int64_t)c->st.n() * c->sn.n() * c->sm.n() * c->sp.n();
@@ -476,6 +479,7 @@ int sed::enqueue_opacity(sed_ctx* c, double dt)
   A.epsilon = c->op.epsilon; A.max_opacity = c->op.maximum_opacity; A.temp_min = c->op.temp_min;
   A.temp_max = c->op.temp_max; A.fleck_alpha = c->tp.fleck_alpha; A.dt = dt; A.time = c->t_now;
   A.nu = dev_loc(c->nu, c->d_nu);
+  A.bin_tab = c->d_bin_tab.p;
   A.rho = c->d_rho.p; A.T = c->d_T.p; A.e_gas = c->d_egas.p; A.grey = c->d_grey.p; A.X = c->d_X.p;
   A.eZ = c->d_eZ.p; A.eA = c->d_eA.p; A.zero_eps_atom = c->d_zero_eps_atom.p;
   A.natoms = c->have_atoms ? c->natoms : 0;
@@ -1115,7 +1119,7 @@ void sed_ctx_destroy(sed_ctx* c)
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
-  DevBuf<double>* dbl[] = {&c->d_nu, &c->d_st, &c->d_sn, &c->d_sm, &c->d_sp, &c->d_core_cdf, &c->d_r_out, &c->d_v_r,
+  DevBuf<double>* dbl[] = {&c->d_nu, &c->d_bin_tab, &c->d_st, &c->d_sn, &c->d_sm, &c->d_sp, &c->d_core_cdf, &c->d_r_out, &c->d_v_r,
                            &c->d_ax[0], &c->d_ax[1], &c->d_ax[2], &c->d_vol, &c->d_rho, &c->d_T, &c->d_egas,
                            &c->d_grey, &c->d_X, &c->d_ion_chi, &c->d_lev_E, &c->d_lev_Eion, &c->d_photo_E,
                            &c->d_photo_s, &c->d_fz_h,

@@ -90,6 +90,7 @@ struct sed_ctx {
   sed_transport_params tp{};
   HostLoc nu, st, sn, sm, sp;
   DevBuf<double> d_nu, d_st, d_sn, d_sm, d_sp, d_core_cdf;
+  DevBuf<double> d_bin_tab;  // zone-independent factors of the frequency bins (launch_bin_table)
   uint32_t step = 0;
 
   // grid

@@ -236,6 +236,7 @@ struct OpacityArgs {
   int32_t radiative_eq, omit_scat, precision;
   double epsilon, max_opacity, temp_min, temp_max, fleck_alpha, dt, time;
   DevLoc nu;
+  const double* bin_tab;                     // [BIN_TAB][n_nu] zone-independent factors of a bin
   const double *rho, *T, *e_gas, *grey, *X;  // zone state
   const int32_t *eZ, *eA;
   const int32_t* zero_eps_atom;  // [nelem] 1 when the atom's epsilon is 0
@@ -286,5 +287,8 @@ size_t opacity_smem_bytes(const OpacityArgs& a);
 // dynamic shared memory of the line-sum kernel (n_pop levels or ions per zone)
 size_t line_sum_smem_bytes(int precision, int natoms, int n_pop);
 int launch_opacity(const OpacityArgs& a, int num_sms, cudaStream_t s);
+// the per-bin factors of a frequency grid, [BIN_TAB][nu.n], once per context
+constexpr int BIN_TAB = 6;
+int launch_bin_table(const DevLoc& nu, double* tab, cudaStream_t s);
 
 }  // namespace sed

@@ -78,3 +78,26 @@ def test_fp64_lte_solve_is_the_same_in_both_forms(sed_lib, monkeypatch):
         g.close()
     for k in ("n_elec", "abs", "scat", "emis_cdf"):
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("n_bins", [2, 33, 300, 1025])
+def test_guide_tables_of_a_build_and_of_a_load_agree(sed_lib, precision, n_bins):
+    """Packets on the tables of a build and on the same tables loaded back
+    (whose guide tables the host forms by binary search) have the same
+    histories to the bit."""
+    n = 1500
+    w = workloads.type_ia(n_packets=n, n_zones=20, n_lines=3000, n_bins=n_bins, seed=5)
+    a = oracle_lib.Engine(sed_lib, "sed_", w, precision=precision)
+    b = oracle_lib.Engine(sed_lib, "sed_", w, precision=precision)
+    a.set_opacity(1.0)
+    t = a.opacity()
+    b.load_opacity(t["abs"], t["scat"], t["emis_cdf"], t["eps_imc"])
+    r = []
+    for e in (a, b):
+        e.record(True)
+        e.transport(1.0)
+        r.append(e.records(n))
+        e.close()
+    for k in ("fate", "ind", "draws", "state"):
+        assert np.array_equal(r[0][k], r[1][k]), k
