@@ -45,6 +45,13 @@
 //  * The frequency bin comes from the FP32 index estimate where it lies
 //    clear of a wall (loc_within_mixed), and after a redistribution from the
 //    interaction itself, with its opacity loaded there.
+//  * One model's kernel reads a re-emission from packed bins, {CDF below, CDF,
+//    abs, scat} in 16 bytes, behind a guide table of eight entries per bin:
+//    two dependent round trips to the L2 instead of four or five, the first
+//    under the direction's arithmetic; eps_imc joins the e_abs sum at the end
+//    of a zone visit instead of being loaded per segment; the Philox key is a
+//    kernel argument (Type Ia packet kernel, 1e6 packets 83.4 -> 78.4 ms, 4e6
+//    232.6 -> 218.2 ms).
 //  * 64 registers, 32 warps per SM: the zone-visit tally sums and the state
 //    a packet reads only at its start or end sit in each thread's slots of
 //    shared memory, and a visit's sums go to one of 32 global tally copies
@@ -126,46 +133,78 @@ __device__ __forceinline__ int next_zone(const StepArgs& A, const GridDev& G, co
   return in_nbr;
 }
 
-// isotropic_scatter (scatter.cpp:303-351) on a homologous flow, with the
-// comoving direction from mu and the azimuth deviate vphi, and (redist) the
-// comoving frequency from the zone's emissivity CDF with deviate word w_cdf
-// Returns the comoving frequency bin of a redistributed photon (-1 for a
-// coherent scatter) and its width times c t in *dnu_num.
-template <typename CT>
-__device__ __forceinline__ int scatter(const StepArgs& A, Pkt& p, double rsq, double xd, double mu, float vphi,
-                                       uint32_t w_cdf, bool redist, float* dnu_num)
+// {abs, scat} of bin k of zone iz, from the packed bins {CDF below, CDF, abs,
+// scat} where the context has them
+__device__ __forceinline__ float2 bin_opacity_pair(const StepArgs& A, int iz, int k)
 {
-  int kbin = -1;
-  const double gamma = rsqrt_nr(fma(-rsq, A.inv_ct2, 1.0));
-  const double dshift_in = gamma * fma(-xd, A.inv_ct, 1.0);
-  p.e = p.e * dshift_in;
-  p.nu = p.nu * dshift_in;
-  float sf, cf;
-  __sincosf(fmaf((float)(2.0 * PI), vphi, -(float)PI), &sf, &cf);
-  const double smu = sqrt_nr(fma(-mu, mu, 1.0));
-  const double Dn0 = smu * (double)cf, Dn1 = smu * (double)sf, Dn2 = mu;
-  if (redist) {  // transport::sample_photon_frequency (emission.cpp:27-46)
-    const int nn = A.nu.n;
-    if (nn == 1) p.nu = loc_sample(A.nu, 0, 0.5);
-    else {
-      const double u = (double)w_cdf * (1.0 / 4294967296.0);
-      int k = cdf_row_sample<CT>(A, p.ind, u);
-      if (k > nn - 1) k = nn - 1;
-      const CT* row = reinterpret_cast<const CT*>(A.cdf) + (size_t)p.ind * nn;
-      const double lo = (k == 0) ? 0.0 : (double)__ldg(row + k - 1);
-      const double hi = (double)__ldg(row + k);
-      float f = __fdividef((float)(u - lo), (float)(hi - lo));
-      f = fminf(fmaxf(f, 0.0f), 0.99999994f);
-      // locate_array::sample (locate_array.cpp:237-242) with the bin's walls
-      // kept for the next segment
-      const double wl = (k == 0) ? A.nu.min : __ldg(A.nu.right + k - 1);
-      const double wr = __ldg(A.nu.right + k);
-      p.nu = wl + (wr - wl) * (double)f;
-      kbin = k;
-      *dnu_num = (float)((wr - wl) * A.ct);
+  const size_t i = (size_t)iz * A.nu.n + k;
+  if (A.bin4) return __ldg(reinterpret_cast<const float2*>(A.bin4 + i) + 1);
+  return __ldg(reinterpret_cast<const float2*>(A.opac) + i);
+}
+
+// a sampled bin: its index, the CDF below and at it, its walls and {abs, scat}
+struct SampledBin {
+  int k;
+  float c0, c1;
+  double2 lr;
+  float2 ab;
+};
+
+// transport::sample_photon_frequency (emission.cpp:27-46): the bin of the
+// zone's emissivity CDF that deviate u selects (upper_bound), from the guide
+// entry `lo` at or below it (one model's kernel).  With the packed bins two
+// neighbouring 16-byte loads, issued together with the walls of both bins, settle almost every u;
+// the rest (guide cells that hold many improbable bins) search up to the next
+// guide entry.
+__device__ __forceinline__ SampledBin sample_bin(const StepArgs& A, int iz, double u, int lo)
+{
+  const int nn = A.nu.n;
+  SampledBin s;
+  if (A.bin4) {
+    const float4* __restrict__ T = A.bin4 + (size_t)iz * nn;
+    int k = min(lo, nn - 1);
+    const int k1 = min(k + 1, nn - 1);
+    float4 v = __ldg(T + k);
+    const float4 v1 = __ldg(T + k1);
+    s.lr = __ldg(A.nu_lr + k);
+    const double2 lr1 = __ldg(A.nu_lr + k1);
+    if ((double)v.y <= u) {
+      k = k1;
+      v = v1;
+      s.lr = lr1;
+      if ((double)v.y <= u) {
+        const uint16_t* g = A.cdf_guide + (size_t)iz * (A.guide_n + 1) + (int)(u * (double)A.guide_n) + 1;
+        int a = min(k + 1, nn - 1), b = min((int)__ldg(g), nn - 1);
+        while (a < b) {
+          const int m = (a + b) >> 1;
+          if ((double)__ldg(&T[m].y) <= u) a = m + 1; else b = m;
+        }
+        k = a;
+        v = __ldg(T + k);
+        s.lr = __ldg(A.nu_lr + k);
+      }
     }
+    s.k = k;
+    s.c0 = v.x;
+    s.c1 = v.y;
+    s.ab = make_float2(v.z, v.w);
+    return s;
   }
-  // comoving -> lab with the velocity reversed, beta = x / (c t)
+  s.k = cdf_row_sample<float>(A, iz, u);
+  if (s.k > nn - 1) s.k = nn - 1;
+  const float* row = reinterpret_cast<const float*>(A.cdf) + (size_t)iz * nn;
+  s.c0 = (s.k == 0) ? 0.f : __ldg(row + s.k - 1);
+  s.c1 = __ldg(row + s.k);
+  s.lr = make_double2((s.k == 0) ? A.nu.min : __ldg(A.nu.right + s.k - 1), __ldg(A.nu.right + s.k));
+  s.ab = __ldg(reinterpret_cast<const float2*>(A.opac) + (size_t)iz * nn + s.k);
+  return s;
+}
+
+// the end of a scatter: the comoving direction Dn, energy and frequency to the
+// lab (lorentz_transform with the velocity reversed)
+__device__ __forceinline__ void to_lab(const StepArgs& A, Pkt& p, double gamma, double Dn0, double Dn1, double Dn2)
+{
+  // beta = x / (c t)
   const double b0 = p.x[0] * A.inv_ct, b1 = p.x[1] * A.inv_ct, b2 = p.x[2] * A.inv_ct;
   const double bdp = -fma(b0, Dn0, fma(b1, Dn1, b2 * Dn2));
   const double vd_out = gamma * (1 - bdp);
@@ -180,10 +219,87 @@ __device__ __forceinline__ int scatter(const StepArgs& A, Pkt& p, double rsq, do
   p.D[2] = D2 * inv_norm;
   p.e = p.e * vd_out;
   p.nu = p.nu * vd_out;
+}
+
+// isotropic_scatter (scatter.cpp:303-351) on a homologous flow, with the
+// comoving direction from mu and the azimuth deviate vphi, and (redist) the
+// comoving frequency from the zone's emissivity CDF with deviate word w_cdf
+// Returns the comoving frequency bin of a redistributed photon (-1 for a
+// coherent scatter), its width times c t in *dnu_num and, in one model's
+// kernel, its {abs, scat} in *ab.
+__device__ __forceinline__ int scatter(const StepArgs& A, Pkt& p, double rsq, double xd, double mu, float vphi,
+                                       uint32_t w_cdf, bool redist, float* dnu_num, float2* ab)
+{
+  const int nn = A.nu.n;
+  const bool look = redist && nn > 1;
+  const double u = (double)w_cdf * (1.0 / 4294967296.0);
+  int lo = 0;  // the guide entry is on its way while the direction's first part is formed
+  if (look && A.bin4) lo = __ldg(A.cdf_guide + (size_t)p.ind * (A.guide_n + 1) + (int)(u * (double)A.guide_n));
+  const double gamma = rsqrt_nr(fma(-rsq, A.inv_ct2, 1.0));
+  const double dshift_in = gamma * fma(-xd, A.inv_ct, 1.0);
+  p.e = p.e * dshift_in;
+  p.nu = p.nu * dshift_in;
+  float sf, cf;
+  __sincosf(fmaf((float)(2.0 * PI), vphi, -(float)PI), &sf, &cf);
+  const double smu = sqrt_nr(fma(-mu, mu, 1.0));
+  const double Dn0 = smu * (double)cf, Dn1 = smu * (double)sf, Dn2 = mu;
+  int kbin = -1;
+  if (look) {
+    const SampledBin s = sample_bin(A, p.ind, u, lo);
+    float f = __fdividef((float)(u - (double)s.c0), (float)((double)s.c1 - (double)s.c0));
+    f = fminf(fmaxf(f, 0.0f), 0.99999994f);
+    // locate_array::sample (locate_array.cpp:237-242) with the bin's width
+    // kept for the next segment
+    const double w = s.lr.y - s.lr.x;
+    p.nu = s.lr.x + w * (double)f;
+    *dnu_num = (float)(w * A.ct);
+    *ab = s.ab;
+    kbin = s.k;
+  } else if (redist) {
+    p.nu = loc_sample(A.nu, 0, 0.5);
+  }
+  to_lab(A, p, gamma, Dn0, Dn1, Dn2);
   return kbin;
 }
 
-// adds one zone visit's tallies: to the block's shared copy [5][nz] when
+// the same for a batch, whose tables spill out of the L2: it reads the 4-byte
+// CDF row (with packed bins its packet kernel ran 148-154 ms against 147)
+__device__ __forceinline__ int scatter_batch(const StepArgs& A, Pkt& p, double rsq, double xd, double mu, float vphi,
+                                             uint32_t w_cdf, bool redist, float* dnu_num)
+{
+  int kbin = -1;
+  const double gamma = rsqrt_nr(fma(-rsq, A.inv_ct2, 1.0));
+  const double dshift_in = gamma * fma(-xd, A.inv_ct, 1.0);
+  p.e = p.e * dshift_in;
+  p.nu = p.nu * dshift_in;
+  float sf, cf;
+  __sincosf(fmaf((float)(2.0 * PI), vphi, -(float)PI), &sf, &cf);
+  const double smu = sqrt_nr(fma(-mu, mu, 1.0));
+  const double Dn0 = smu * (double)cf, Dn1 = smu * (double)sf, Dn2 = mu;
+  if (redist) {
+    const int nn = A.nu.n;
+    if (nn == 1) p.nu = loc_sample(A.nu, 0, 0.5);
+    else {
+      const double u = (double)w_cdf * (1.0 / 4294967296.0);
+      int k = cdf_row_sample<float>(A, p.ind, u);
+      if (k > nn - 1) k = nn - 1;
+      const float* row = reinterpret_cast<const float*>(A.cdf) + (size_t)p.ind * nn;
+      const double lo = (k == 0) ? 0.0 : (double)__ldg(row + k - 1);
+      const double hi = (double)__ldg(row + k);
+      float f = __fdividef((float)(u - lo), (float)(hi - lo));
+      f = fminf(fmaxf(f, 0.0f), 0.99999994f);
+      const double wl = (k == 0) ? A.nu.min : __ldg(A.nu.right + k - 1);
+      const double wr = __ldg(A.nu.right + k);
+      p.nu = wl + (wr - wl) * (double)f;
+      kbin = k;
+      *dnu_num = (float)((wr - wl) * A.ct);
+    }
+  }
+  to_lab(A, p, gamma, Dn0, Dn1, Dn2);
+  return kbin;
+}
+
+// adds one zone visit's tallies (the e_abs sum times the zone's eps_imc): to the block's shared copy [5][nz] when
 // A.smem_zones, else to global copy rep_off / (5 nz) of the n_rep copies
 // (rep_off < 0: the arrays themselves).  The targets are formed here, from
 // the shared array and the kernel's arguments, rather than held as five
@@ -228,6 +344,25 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem)
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// The packet's stream (PacketRng::block).  One model's key and step number
+// are the kernel's arguments, so the ten round keys are warp-uniform values
+// and neither takes a register; a batch's key is its model's.
+template <int BATCH>
+struct Stream : PacketRng {
+  __device__ __forceinline__ uint4 block(const StepArgs&) { return PacketRng::block(); }
+};
+template <>
+struct Stream<0> {
+  uint64_t pid;
+  uint32_t n;
+  __device__ __forceinline__ void init(uint32_t, uint64_t pid_, uint32_t, uint32_t n0) { pid = pid_; n = n0; }
+  __device__ __forceinline__ uint4 block(const StepArgs& A)
+  {
+    const PhiloxOut o = philox4x32_10(n++, (uint32_t)pid, (uint32_t)(pid >> 32), A.step, A.seed, 1u);
+    return make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
+  }
+};
 
 // the state emit_mixed_kernel stored for core packet q
 __device__ __forceinline__ void load_emitted(const StepArgs& A, Pkt& p, int64_t q)
@@ -296,7 +431,6 @@ template <int BATCH, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const StepArgs A, const GridDev G)
 {
   using namespace mixed;
-  using CT = float;
   extern __shared__ double s_tal[];  // [5][nz] when A.smem_zones
   // the block's event counters, added to once per packet (escaped, absorbed,
   // stopped, segments, interactions, segment-limit stops)
@@ -315,7 +449,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
   uint32_t step = A.step;
   if constexpr (BATCH) step = *A.step_dev;
   Pkt p;
-  PacketRng rng;
+  Stream<BATCH> rng;
   int fate = ABSORBED;  // no packet yet
   bool have = false;
   int32_t seg = 0;
@@ -354,7 +488,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
   __shared__ int s_oz[SLOTS == 2 ? THREADS : 1];
   auto flush_slot = [&](int z, int k) {  // send slot k's sums for zone z and zero the slot
     double* a = &s_acc[k][0][tid];
-    add_visit(A, s_tal, nz, rep_off, z, a[0], a[THREADS], a[2 * THREADS], a[3 * THREADS], a[4 * THREADS]);
+    add_visit(A, s_tal, nz, rep_off, z, a[0] * __ldg(A.eps_imc + z), a[THREADS], a[2 * THREADS], a[3 * THREADS], a[4 * THREADS]);
     a[0] = 0.0; a[THREADS] = 0.0; a[2 * THREADS] = 0.0; a[3 * THREADS] = 0.0; a[4 * THREADS] = 0.0;
   };
   for (int k = 0; k < SLOTS; ++k)
@@ -467,7 +601,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
           p.ind = A.q_ind[k];
           rng.init(A.seed, (uint64_t)(A.radio_first_pid + k), step, qn);
           s_k0[tid] = 0;
-          tau_rem = neg_log_u(rng.block().x);
+          tau_rem = neg_log_u(rng.block(A).x);
         } else {
           rng.init(A.seed, (uint64_t)A.first_pid + pid, step, K_core);  // after the emission's blocks
           s_k0[tid] = K_core;
@@ -533,8 +667,14 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
       nxt_bin = -1;
     } else {
       i_nu = loc_within_mixed(A.nu, p.nu * dshift);
-      ab = __ldg(opac + (size_t)iz * nn + i_nu);
-      dnu_num = (float)(loc_delta(A.nu, i_nu) * A.ct);
+      if constexpr (BATCH) {
+        ab = __ldg(opac + (size_t)iz * nn + i_nu);
+        dnu_num = (float)(loc_delta(A.nu, i_nu) * A.ct);
+      } else {
+        ab = bin_opacity_pair(A, iz, i_nu);
+        const double2 w = __ldg(A.nu_lr + i_nu);
+        dnu_num = (float)((w.y - w.x) * A.ct);
+      }
     }
     const float a_f = ab.x;
     const float s_f = A.omit_scat ? 0.0f : ab.y;
@@ -555,10 +695,12 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
     else { event = 2; this_d = d_tm; }
     // tallies (transport.cpp:361-392)
     const double this_E = p.e * this_d;
-    const double eps_imc = __ldg(A.eps_imc + iz);
+    double eps_imc = 1.0;
+    if constexpr (BATCH) eps_imc = __ldg(A.eps_imc + iz);
     const double ed = this_E * dshift;
     double* sa = &s_acc[SLOTS == 2 ? (acc & 1) : 0][0][tid];
-    sa[0] = fma(ed * dshift * (double)a_f, eps_imc, sa[0]);
+    if constexpr (BATCH) sa[0] = fma(ed * dshift * (double)a_f, eps_imc, sa[0]);
+    else sa[0] = fma(ed * dshift, (double)a_f, sa[0]);  // times eps_imc at the flush: no load per segment
     atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
     if (A.tally_forces) {
       const double wd = ed * (double)op_f * dshift;
@@ -589,7 +731,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
     } else if (event == 0) {
       // do_scatter (scatter.cpp:12-70): u <= eps is the absorption branch;
       // the deviate left over from each test is recycled into the next
-      const uint4 blk = rng.block();
+      const uint4 blk = rng.block(A);
       tau_rem = neg_log_u(blk.x);  // the next flight's depth
       const float u1 = (float)blk.y * W32;
       const float num = u1 * op_f;
@@ -599,7 +741,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
         v = __fdividef(num, a_f);
         redist = true;
         if (!A.radiative_eq) {
-          const float ei = (float)eps_imc;
+          const float ei = (float)(BATCH ? eps_imc : __ldg(A.eps_imc + iz));
           if (v > ei) v = __fdividef(v - ei, 1.0f - ei);  // effective scattering
           else { fate = ABSORBED; redist = false; }
         }
@@ -608,16 +750,19 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
       }
       if (fate == MOVING) {
         const double mu = 1.0 - 2.0 * ((double)blk.w * (1.0 / 4294967296.0));
+        const float vphi = fminf(fmaxf(v, 0.0f), 1.0f);
         float dnu_new = 0.f;
-        nxt_bin = scatter<CT>(A, p, rsq, xd, mu, fminf(fmaxf(v, 0.0f), 1.0f), blk.z, redist, &dnu_new);
-        if (nxt_bin >= 0) {  // the new bin's {abs, scat}, loaded ahead of its use
-          if constexpr (BATCH) {
+        if constexpr (BATCH) {  // the new bin's {abs, scat}, on its way to the slot the next segment reads
+          nxt_bin = scatter_batch(A, p, rsq, xd, mu, vphi, blk.z, redist, &dnu_new);
+          if (nxt_bin >= 0) {
             cp_async8(s_nab + tid, opac + (size_t)iz * nn + nxt_bin);
             s_ndnu[tid] = dnu_new;
-          } else {
-            nxt_ab = __ldg(opac + (size_t)iz * nn + nxt_bin);
-            nxt_dnu = dnu_new;
           }
+        } else {
+          float2 ab_new = make_float2(0.f, 0.f);
+          nxt_bin = scatter(A, p, rsq, xd, mu, vphi, blk.z, redist, &dnu_new, &ab_new);
+          nxt_ab = ab_new;
+          nxt_dnu = dnu_new;
         }
         xd = fma(p.D[0], p.x[0], fma(p.D[1], p.x[1], p.D[2] * p.x[2]));
       }
@@ -625,7 +770,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
       fate = STOPPED;
     }
   }
-  cp_async_wait();
+  if constexpr (BATCH) cp_async_wait();
   __syncthreads();
   if (threadIdx.x < 6) {
     constexpr int slot[6] = {C_ESCAPED, C_ABSORBED, C_STOPPED, C_SEGMENTS, C_SCATTERS, C_LIMIT};

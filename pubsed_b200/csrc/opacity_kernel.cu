@@ -643,17 +643,45 @@ __global__ void __launch_bounds__(32 * LINE_SUM_WARPS) line_sum_kernel(const Opa
 // and a handful of divisions instead of a pow() and a dozen divisions more.
 enum BinTab { BT_NU, BT_B, BT_HNK, BT_NU4, BT_D, BT_FAC };
 
-__global__ void bin_table_kernel(const DevLoc nu_grid, double* __restrict__ tab)
+__global__ void bin_table_kernel(const DevLoc nu_grid, double* __restrict__ tab, double2* __restrict__ lr)
 {
   const int nn = nu_grid.n;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nn; j += gridDim.x * blockDim.x) {
     const double nu = loc_center(nu_grid, j), d = loc_delta(nu_grid, j);
+    lr[j] = make_double2(loc_left(nu_grid, j), nu_grid.right[j]);
     tab[BT_NU * nn + j] = nu;
     tab[BT_B * nn + j] = 2.0 * nu * nu * nu * H_PLANCK / C_LIGHT / C_LIGHT;  // B_nu (e^zeta - 1)
     tab[BT_HNK * nn + j] = H_PLANCK * nu / K_BOLTZ;                          // zeta T
     tab[BT_NU4 * nn + j] = pow(nu, 4);
     tab[BT_D * nn + j] = d;
     tab[BT_FAC * nn + j] = nu / d / C_LIGHT;  // times 1/t: the expansion opacity of one Sobolev term
+  }
+}
+
+// the guide tables of zone_opacity_kernel, from CDF rows written otherwise
+template <typename T>
+__global__ void guide_kernel(const T* __restrict__ cdf, int64_t nz, int nn, uint16_t* __restrict__ guide, int G)
+{
+  const int64_t n = nz * (G + 1);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const T* row = cdf + (size_t)(i / (G + 1)) * nn;
+    const double t = (double)(i % (G + 1)) / (double)G;
+    int lo = 0, hi = nn;
+    while (lo < hi) {
+      const int m = (lo + hi) >> 1;
+      if ((double)row[m] <= t) lo = m + 1; else hi = m;
+    }
+    guide[i] = (uint16_t)lo;
+  }
+}
+
+// the packed bins of zone_opacity_kernel, from tables written otherwise
+__global__ void pack_bins_kernel(const float2* __restrict__ opac, const float* __restrict__ cdf, int64_t n, int nn,
+                                 float4* __restrict__ out)
+{
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float2 o = opac[i];
+    out[i] = make_float4(i % nn ? cdf[i - 1] : 0.f, cdf[i], o.x, o.y);
   }
 }
 
@@ -985,10 +1013,15 @@ __global__ void __launch_bounds__(THREADS, BF ? 1 : 1024 / THREADS) zone_opacity
   // nn from k = G on: each bin writes the entries it owns, G + 1 in all,
   // instead of a binary search of the row for every entry.  Any other row
   // (an overflowed or a falling one) is searched.
+  __syncthreads();
+  if constexpr (MIXED)
+    if (A.bin4_out)
+      for (int j = tid; j < nn; j += bd)
+        A.bin4_out[(size_t)z * nn + j] =
+            make_float4(j ? (float)em[j - 1] : 0.f, (float)em[j], (float)ab_r[j], (float)sc_r[j]);
   if (A.cdf_guide_out) {
     const int G = A.guide_n;
     uint16_t* gz = A.cdf_guide_out + (size_t)z * (G + 1);
-    __syncthreads();
     bool rises = true;
     for (int j = tid; j < nn; j += bd) rises = rises && ((j ? em[j - 1] : 0.0) <= em[j]) && em[j] <= 1.0;
     if (__syncthreads_and(rises && em[nn - 1] == 1.0)) {
@@ -1043,9 +1076,25 @@ int launch_line_sums(const OpacityArgs& a, double* S, double* Se, int num_sms, c
 
 }  // namespace
 
-int launch_bin_table(const DevLoc& nu, double* tab, cudaStream_t s)
+int launch_bin_table(const DevLoc& nu, double* tab, double2* lr, cudaStream_t s)
 {
-  bin_table_kernel<<<(nu.n + 127) / 128, 128, 0, s>>>(nu, tab);
+  bin_table_kernel<<<(nu.n + 127) / 128, 128, 0, s>>>(nu, tab, lr);
+  return 1;
+}
+
+int launch_guide(int precision, const void* cdf, int64_t nz, int nn, uint16_t* guide, int G, int num_sms,
+                 cudaStream_t s)
+{
+  const unsigned b = (unsigned)num_sms * 8;
+  if (precision) guide_kernel<<<b, 256, 0, s>>>(static_cast<const float*>(cdf), nz, nn, guide, G);
+  else guide_kernel<<<b, 256, 0, s>>>(static_cast<const double*>(cdf), nz, nn, guide, G);
+  return 1;
+}
+
+int launch_pack_bins(const void* opac, const void* cdf, int64_t nz, int nn, float4* out, int num_sms, cudaStream_t s)
+{
+  pack_bins_kernel<<<num_sms * 8, 256, 0, s>>>(static_cast<const float2*>(opac), static_cast<const float*>(cdf),
+                                               nz * nn, nn, out);
   return 1;
 }
 

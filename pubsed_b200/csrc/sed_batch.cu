@@ -146,6 +146,7 @@ StepArgs step_args(sed_batch* b, double dt, const BatchModel* models, int64_t to
   A.a3 = c->sp.n(); A.a2 = (int64_t)c->sm.n() * A.a3; A.a1 = (int64_t)c->sn.n() * A.a2;
   A.opac = c->d_opac.p; A.cdf = c->d_cdf.p; A.eps_imc = c->d_eps_imc.p;
   A.cdf_coarse = c->d_cdf_coarse.p; A.n_coarse = c->n_coarse;
+  A.nu_lr = c->d_nu_lr.p;
   A.cdf_guide = c->guide_n ? c->d_cdf_guide.p : nullptr; A.guide_n = c->guide_n;
   A.rescale_lum = c->tp.core_fix_luminosity;
   A.J = c->d_J.p; A.e_abs = c->d_e_abs.p; A.e_rad = c->d_e_rad.p;
@@ -246,6 +247,7 @@ int sed_batch_create(const sed_transport_params* common, double t_now, int32_t n
   int rc = sed_ctx_create(common, device, &b->inner);
   if (rc) { delete b; return rc; }
   sed_ctx* c = b->inner;
+  c->in_batch = true;
   // concatenated zone arrays: the inner context's grid
   std::vector<double> r_out, vol, rho, T, eg, grey, X;
   std::vector<int4> nbr;

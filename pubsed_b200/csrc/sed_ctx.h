@@ -127,6 +127,9 @@ struct sed_ctx {
   bool opac_base_valid = false;       // d_opac_base holds the tables of the last build or load
   bool opac_scaled = false;           // d_opac holds density-scaled tables
   int n_coarse = 0;
+  bool in_batch = false;         // the inner context of a batch
+  DevBuf<float4> d_bin4;         // packed bins of the 1D mixed packet kernel (FP32 tables on 1D grids)
+  DevBuf<double2> d_nu_lr;       // {left, right} walls of the frequency bins
   DevBuf<uint16_t> d_cdf_guide;  // CDF guide tables, guide_n + 1 entries per zone
   int guide_n = 0;
   int chunk_zones = 0;  // zones per opacity-build pass (bounds the FP64/LTE scratch)
@@ -252,6 +255,8 @@ inline bool valid_grid(const sed_locate_grid& g) { return g.n > 0 && g.right != 
 int enqueue_opacity(sed_ctx* c, double dt);
 
 // kernel arguments and device grid of a transport step of this context
+// the packed bins again, after the {abs, scat} or CDF tables were written by something else than an opacity build
+cudaError_t pack_bins(sed_ctx* c);
 StepArgs make_step_args(sed_ctx* c, double dt, int64_t n_emit);
 GridDev make_grid_dev(sed_ctx* c);
 

@@ -273,6 +273,7 @@ int scale_extinction(sed_ctx* c, const double* r, cudaMemcpyKind in)
     CK(cudaGetLastError());
     c->opac_scaled = true;
   }
+  CK(pack_bins(c));
   CK(cudaStreamSynchronize(c->stream));
   return SED_OK;
 }

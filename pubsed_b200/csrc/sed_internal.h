@@ -46,6 +46,8 @@ struct StepArgs {
   int64_t a1, a2, a3;         // spectrum strides
   const void* opac;           // [nz*n_nu] double2 {abs, scat} or float2
   const void* cdf;            // [nz*n_nu] double or float emissivity CDF
+  const float4* bin4;         // [nz*n_nu] {CDF below, CDF, abs, scat} of a bin (FP32 tables on 1D grids), or null
+  const double2* nu_lr;       // [n_nu] {left, right} wall of a frequency bin
   const void* cdf_coarse;     // [nz*n_coarse] every CDF_STRIDE-th CDF value (last of each block)
   int32_t n_coarse;           // blocks per zone row = ceil(n_nu / CDF_STRIDE)
   const uint16_t* cdf_guide;  // [nz*(guide_n+1)] guide[k] = upper_bound(CDF row, k / guide_n), or null
@@ -275,6 +277,7 @@ struct OpacityArgs {
   double *epsl64, *epsf64;               // [nz*n_nu] epsilon-weighted line / fuzz sums (same condition)
   void* opac_out;                        // double2 / float2 [nz*n_nu]
   void* cdf_out;                         // double / float [nz*n_nu]
+  float4* bin4_out;                      // [nz*n_nu] {CDF below, CDF, abs, scat} (FP32 tables), or null
   void* cdf_coarse_out;                  // double / float [nz*n_coarse]
   int32_t n_coarse;
   uint16_t* cdf_guide_out;               // [nz*(guide_n+1)] or null
@@ -289,6 +292,11 @@ size_t line_sum_smem_bytes(int precision, int natoms, int n_pop);
 int launch_opacity(const OpacityArgs& a, int num_sms, cudaStream_t s);
 // the per-bin factors of a frequency grid, [BIN_TAB][nu.n], once per context
 constexpr int BIN_TAB = 6;
-int launch_bin_table(const DevLoc& nu, double* tab, cudaStream_t s);
+int launch_bin_table(const DevLoc& nu, double* tab, double2* lr, cudaStream_t s);
+// guide tables of stored CDF rows (FP32 or FP64): guide[k] = upper_bound(row, k / G)
+int launch_guide(int precision, const void* cdf, int64_t nz, int nn, uint16_t* guide, int G, int num_sms,
+                 cudaStream_t s);
+// the {CDF below, CDF, abs, scat} table from FP32 {abs, scat} pairs and CDF rows
+int launch_pack_bins(const void* opac, const void* cdf, int64_t nz, int nn, float4* out, int num_sms, cudaStream_t s);
 
 }  // namespace sed
