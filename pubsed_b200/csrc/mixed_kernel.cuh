@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
   Walls wl{};
   double rsq = 0, xd = 0;
   float tau_rem = 0;  // optical depth left to the next interaction
-  bool live = true;   // the lane still takes packets from the queue
+  bool live = (int)(threadIdx.x & 31) < A.lanes;  // the lane still takes packets from the queue
   // after a redistribution: the photon's comoving bin (its lab frequency
   // transforms back into that bin at the next segment's start, which is the
   // interaction point), its {abs, scat}, loaded ahead, and its width times

@@ -136,12 +136,7 @@ StepArgs sed::make_step_args(sed_ctx* c, double dt, int64_t n_emit)
   A.first_pid = c->tp.first_packet_id;
   A.Ep = n_emit > 0 ? c->tp.core_luminosity * dt / n_emit : 0.0;
   A.t_now = c->t_now; A.dt = dt; A.tstop = c->t_now + dt;
-  if (c->t_grid > 0) {
-    A.inv_t = 1.0 / c->t_grid;
-    A.ct = C_LIGHT * c->t_grid;
-    A.inv_ct = 1.0 / A.ct;
-    A.inv_ct2 = A.inv_ct * A.inv_ct;
-  }
+  set_grid_time(A, c->t_grid);
   A.core_radius = c->tp.core_radius; A.core_freq = c->tp.core_photon_frequency; A.core_cdf = c->d_core_cdf.p;
   A.max_segments = c->tp.max_segments;
   A.use_ddmc = c->tp.use_ddmc; A.ddmc_tau = c->tp.ddmc_tau;
@@ -802,8 +797,8 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
     CK(c->d_em_tau.resize((size_t)n_emit));
     A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_tau = c->d_em_tau.p; A.em_n = n_emit;
   }
-  if (mixed_1d_path(A, G)) {
-    // the 1D mixed kernel adds each zone visit's tallies to one of n_rep
+  if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G))) {
+    // the 1D packet kernels of homologous grids add each zone visit's tallies to one of n_rep
     // global copies (block b to copy b % n_rep, fire-and-forget reductions),
     // which the finish kernel sums: against the per-block shared-memory
     // copies, whose atomic adds hold the warp, the Type Ia packet kernel ran

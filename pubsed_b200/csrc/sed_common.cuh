@@ -145,6 +145,70 @@ __device__ __forceinline__ double rcp_nr(double a)
   return fma(y, fma(e, e, e), y);              // y (1 + e + e^2)
 }
 
+// ------------------------------------------- IEEE results without branches
+// Division, reciprocal and square root rounded as IEEE 754 rounds them, for
+// operands and results in the normal range (and a zero dividend or radicand),
+// as straight-line code: CUDA's own branch to a special-case path, and the
+// compiler overlaps nothing across those branches.  The methods are
+// Markstein's (IA-64 and Elementary Functions, 2000, chapters 8 and 9): a
+// reciprocal within an ulp of 1/b becomes the rounded one by one more Newton
+// step with an exact residual, a quotient (root) within an ulp becomes the
+// rounded one by one correction with an exact residual.  Both theorems except
+// a divisor whose 53 bits are all ones.
+
+// 1/b
+__device__ __forceinline__ double rcp_rn(double b)
+{
+  const double y = rcp_nr(b);
+  return fma(fma(-b, y, 1.0), y, y);
+}
+
+// a/b from y = rcp_rn(b)
+__device__ __forceinline__ double div_rn(double a, double b, double y)
+{
+  const double q0 = a * y;                         // within two ulp
+  const double q1 = fma(fma(-b, q0, a), y, q0);    // within one
+  return fma(fma(-b, q1, a), y, q1);
+}
+__device__ __forceinline__ double div_rn(double a, double b) { return div_rn(a, b, rcp_rn(b)); }
+
+// sqrt(a), and y = 1/sqrt(a) to about an ulp (a > 0)
+__device__ __forceinline__ double sqrt_rn(double a, double* y)
+{
+  const double r = rsqrt_nr(a), h = 0.5 * r;
+  const double s0 = a * r;
+  const double s1 = fma(fma(-s0, s0, a), h, s0);
+  const double s2 = fma(fma(-s1, s1, a), h, s1);
+  *y = r;
+  return s2;
+}
+__device__ __forceinline__ double sqrt_rn(double a)
+{
+  double y;
+  const double s = sqrt_rn(a, &y);
+  return (a == 0.0) ? a : s;
+}
+// 1.0 / sqrt(a), both rounded, a > 0
+__device__ __forceinline__ double rcp_sqrt_rn(double a)
+{
+  double y;
+  const double s = sqrt_rn(a, &y);
+  return fma(fma(-s, y, 1.0), y, y);
+}
+
+// a/b for a divisor known ahead, zh + zl its reciprocal to twice the precision
+// (Brisebarre, Muller and Raina, IEEE Trans. Computers 53, 2004): the quotient
+// is off by hardly more than half an ulp, then corrected as above
+__host__ __device__ __forceinline__ double div_by(double a, double b, double zh, double zl)
+{
+  const double q = fma(a, zh, a * zl);
+  return fma(fma(-b, q, a), zh, q);
+}
+__device__ __forceinline__ double div_c(double a)  // by the speed of light
+{
+  return div_by(a, C_LIGHT, 0x1.2567f4ed09fe8p-35, 0x1.b54b6f1e0ba5ep-89);
+}
+
 // ---------------------------------------------------------------- locate
 struct DevLoc {
   int32_t n, type;

@@ -33,6 +33,8 @@ struct StepArgs {
   int64_t first_pid;          // Philox stream id of queue entry 0
   double Ep, t_now, dt, tstop;
   double inv_t, ct, inv_ct, inv_ct2;  // 1/t_grid, c t_grid, 1/(c t_grid), its square (homologous flow)
+  double t_grid, inv_t_lo;            // grid time; 1/t_grid - inv_t
+  double inv_dvds, inv_dvds_lo;       // 1/inv_t and what its rounding left (the FP64 kernel divides by inv_t)
   double core_radius, core_freq;
   const double* core_cdf;     // [n_nu] normalised core emission CDF
   int32_t max_segments;
@@ -54,7 +56,7 @@ struct StepArgs {
   int32_t guide_n;            // power of two >= n_nu (0: no guide table, n_nu > 65535)
   const double* eps_imc;      // [nz]
   int32_t rescale_lum;        // core_fix_luminosity (steady-state rescale)
-  int32_t pad_;
+  int32_t lanes;              // lanes of a warp that take packets (32, fewer for few packets; launch_* set it)
   double* J;                  // [nz * (store_Jnu ? n_nu : 1)]
   double *e_abs, *e_rad, *fx, *fy, *fz, *fr;
   double *flux, *click;
@@ -189,12 +191,16 @@ struct BatchModel {
   const double* core_cdf;            // [n_nu] normalised core emission CDF
 };
 
+// the grid-time factors of a step's arguments: 1/t, c t and their like
+void set_grid_time(StepArgs& a, double t_grid);
 // launches the persistent packet kernel; returns the number of launches
 int launch_propagate(const StepArgs& a, const GridDev& g, int num_sms, cudaStream_t s);
 // whether launch_propagate runs the mixed-form 1D kernel for these
 // arguments: its core packets are then emitted ahead into the em_* buffers
 // (A.em_n of them), which the caller provides
 bool mixed_1d_path(const StepArgs& a, const GridDev& g);
+// whether it runs the FP64 kernel of homologous grids (fp64_kernel.cuh)
+bool fp64_path(const StepArgs& a, const GridDev& g);
 // IMD probabilities of the step (transport::compute_diffusion_probabilities)
 // from the zone Planck means into out[4][nz]
 int launch_imd_probabilities(const GridDev& g, const double* planck, double dt, double* out, cudaStream_t s);

@@ -15,6 +15,7 @@
 // compiled without FMA contraction so products and sums round as written.
 #include <cfloat>
 #include <cmath>
+#include <algorithm>
 #include "sed_internal.h"
 
 namespace sed {
@@ -1886,6 +1887,28 @@ __global__ void init_particles_kernel(const InitArgs I, const GridDev G)
 }
 
 #include "mixed_kernel.cuh"
+#include "fp64_kernel.cuh"
+
+// Blocks of a persistent packet kernel, `per_sm` of which fit on an SM, and
+// the lanes of a warp that take packets.  With fewer packets than the chip has
+// lanes a step lasts as long as its longest packet's chain of segments, and a
+// warp of 32 packets walks every branch any of them takes: up to
+// SPREAD_WARPS_PER_SM warps per SM (four per scheduler, which leaves each a
+// warp's own latency) get equal shares of the packets instead of the first
+// blocks 32 to a warp.  2000 packets of the grey lightbulb (FP64) 3.28 -> 2.48
+// ms, 2e4 3.74 -> 3.46 ms, 2e4 of the 97-zone line model (mixed) 4.94 -> 4.5 ms;
+// 8 and 12 warps per SM 2.44 and 2.47, 3.51 and 3.45, 4.7 and 4.6 ms, 32 no gain.
+constexpr int SPREAD_WARPS_PER_SM = 16;
+
+int64_t spread_packets(int64_t total, int threads, int per_sm, int num_sms, int32_t* lanes)
+{
+  const int64_t resident = (int64_t)num_sms * per_sm;
+  const int64_t warps = std::min<int64_t>((int64_t)num_sms * SPREAD_WARPS_PER_SM, resident * (threads / 32));
+  const int64_t l = std::min<int64_t>(32, std::max<int64_t>(1, (total + warps - 1) / warps));
+  *lanes = (int32_t)l;
+  const int64_t per_block = l * (threads / 32);
+  return std::max<int64_t>(1, std::min(resident, (total + per_block - 1) / per_block));
+}
 
 // the mixed-form 1D kernel (propagate_mixed_kernel) in one compiled shape
 // (zone-scalar tallies go to global memory when MINB blocks' shared-memory
@@ -1912,12 +1935,25 @@ int launch_mixed_t(const StepArgs& a0, const GridDev& g, int blocks_per_sm, int 
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem);
   if (per_sm < 1) per_sm = 1;
   if (blocks_per_sm > 0 && blocks_per_sm < per_sm) per_sm = blocks_per_sm;
-  int64_t blocks = (int64_t)num_sms * per_sm;
-  const int64_t need = (total + THREADS - 1) / THREADS;
-  if (blocks > need) blocks = need;
-  if (blocks < 1) blocks = 1;
+  const int64_t blocks = spread_packets(total, THREADS, per_sm, num_sms, &a.lanes);
   kern<<<(unsigned)blocks, THREADS, smem, s>>>(a, g);
   return a.em_n > 0 ? 2 : 1;
+}
+
+template <int GRID, int BATCH, int THREADS, int MINB>
+int launch_fp64_t(const StepArgs& a0, const GridDev& g, int blocks_per_sm, int num_sms, int64_t total, cudaStream_t s)
+{
+  StepArgs a = a0;
+  const size_t smem = a.smem_zones ? (size_t)5 * g.nzones * sizeof(double) : 0;
+  auto kern = propagate_fp64_kernel<GRID, BATCH, THREADS, MINB>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem);
+  if (per_sm < 1) per_sm = 1;
+  if (blocks_per_sm > 0 && blocks_per_sm < per_sm) per_sm = blocks_per_sm;
+  const int64_t blocks = spread_packets(total, THREADS, per_sm, num_sms, &a.lanes);
+  kern<<<(unsigned)blocks, THREADS, smem, s>>>(a, g);
+  return 1;
 }
 
 template <int GRID, typename OT, typename CT, int BATCH, int THREADS, int MINB, int MODE = 0,
@@ -1945,6 +1981,12 @@ int launch_kernel_t(const StepArgs& a, const GridDev& g, int blocks_per_sm, int 
 // 1D grids is propagate_mixed_kernel (SED_MIXED_THREADS x SED_MIXED_MINB);
 // on 3D grids the mixed form runs 128 x 7 (64^3 cells, 2e7 packets: packet
 // kernel 572 ms vs 583 ms at 256 x 3).
+// the FP64 kernel's grids: homologous, at a time its reciprocals cover
+bool fp64_ok(const StepArgs& a, const GridDev& g)
+{
+  return a.precision == 0 && g.homologous && a.use_ddmc == 0 && a.t_grid > 1e-100 && a.t_grid < 1e100;
+}
+
 template <int GRID, typename OT, typename CT>
 int launch_propagate_t(const StepArgs& a, const GridDev& g, int num_sms, cudaStream_t s)
 {
@@ -1961,6 +2003,14 @@ int launch_propagate_t(const StepArgs& a, const GridDev& g, int num_sms, cudaStr
     if constexpr (GRID == 0) return launch_mixed_t<0, SED_MIXED_THREADS, SED_MIXED_MINB>(a, g, 0, num_sms, a.n_packets, s);
     else return launch_kernel_t<GRID, OT, CT, 0, 128, 7>(a, g, 0, num_sms, a.n_packets, s);
   } else {
+    if (fp64_ok(a, g)) {
+      // few packets wait for the longest chain: 16 warps per SM at 112
+      // registers; many fill the SM: 24 warps at 80 (Type Ia, packet kernel:
+      // 3e5 packets 92 against 108 ms, 1e6 151 against 158, 2e6 274 against
+      // 241 ms; grey lightbulb 1e5 6.5 against 7.1, 1e6 31.0 against 28.0 ms)
+      if (a.n_packets < (int64_t)num_sms * 768 * 8) return launch_fp64_t<GRID, 0, 128, 4>(a, g, 0, num_sms, a.n_packets, s);
+      return launch_fp64_t<GRID, 0, 256, 3>(a, g, 0, num_sms, a.n_packets, s);
+    }
     return launch_kernel_t<GRID, OT, CT, 0, 256, 4>(a, g, 0, num_sms, a.n_packets, s);
   }
 }
@@ -1981,11 +2031,12 @@ int launch_batch_t(const StepArgs& a, const GridDev& g, int variant, int bps, in
       default: return launch_mixed_t<1, BATCH_SHAPES[0][0], BATCH_SHAPES[0][1]>(a, g, bps, num_sms, total, s);
     }
   } else {
+    if (!fp64_ok(a, g)) return launch_kernel_t<0, OT, CT, 1, 256, 4>(a, g, bps, num_sms, total, s);
     switch (variant) {
-      case 1: return launch_kernel_t<0, OT, CT, 1, BATCH_SHAPES[1][0], BATCH_SHAPES[1][1]>(a, g, bps, num_sms, total, s);
-      case 2: return launch_kernel_t<0, OT, CT, 1, BATCH_SHAPES[2][0], BATCH_SHAPES[2][1]>(a, g, bps, num_sms, total, s);
-      case 3: return launch_kernel_t<0, OT, CT, 1, BATCH_SHAPES[3][0], BATCH_SHAPES[3][1]>(a, g, bps, num_sms, total, s);
-      default: return launch_kernel_t<0, OT, CT, 1, BATCH_SHAPES[0][0], BATCH_SHAPES[0][1]>(a, g, bps, num_sms, total, s);
+      case 1: return launch_fp64_t<0, 1, BATCH_SHAPES[1][0], BATCH_SHAPES[1][1]>(a, g, bps, num_sms, total, s);
+      case 2: return launch_fp64_t<0, 1, BATCH_SHAPES[2][0], BATCH_SHAPES[2][1]>(a, g, bps, num_sms, total, s);
+      case 3: return launch_fp64_t<0, 1, BATCH_SHAPES[3][0], BATCH_SHAPES[3][1]>(a, g, bps, num_sms, total, s);
+      default: return launch_fp64_t<0, 1, BATCH_SHAPES[0][0], BATCH_SHAPES[0][1]>(a, g, bps, num_sms, total, s);
     }
   }
 }
@@ -1995,6 +2046,22 @@ int launch_batch_t(const StepArgs& a, const GridDev& g, int variant, int bps, in
 bool mixed_1d_path(const StepArgs& a, const GridDev& g)
 {
   return a.precision != 0 && g.type == 0 && g.homologous && a.use_ddmc == 0;
+}
+
+bool fp64_path(const StepArgs& a, const GridDev& g) { return fp64_ok(a, g); }
+
+void set_grid_time(StepArgs& a, double t_grid)
+{
+  a.t_grid = t_grid;
+  if (!(t_grid > 0)) return;
+  a.inv_t = 1.0 / t_grid;
+  a.ct = C_LIGHT * t_grid;
+  a.inv_ct = 1.0 / a.ct;
+  a.inv_ct2 = a.inv_ct * a.inv_ct;
+  // what the rounding of a reciprocal left, relative to it: (1 - b z) z
+  a.inv_t_lo = std::fma(-t_grid, a.inv_t, 1.0) * a.inv_t;
+  a.inv_dvds = 1.0 / a.inv_t;
+  a.inv_dvds_lo = std::fma(-a.inv_t, a.inv_dvds, 1.0) * a.inv_dvds;
 }
 
 int launch_propagate(const StepArgs& a, const GridDev& g, int num_sms, cudaStream_t s)
