@@ -48,10 +48,11 @@
 //  * One model's kernel reads a re-emission from packed bins, {CDF below, CDF,
 //    abs, scat} in 16 bytes, behind a guide table of eight entries per bin:
 //    two dependent round trips to the L2 instead of four or five, the first
-//    under the direction's arithmetic; eps_imc joins the e_abs sum at the end
-//    of a zone visit instead of being loaded per segment; the Philox key is a
-//    kernel argument (Type Ia packet kernel, 1e6 packets 83.4 -> 78.4 ms, 4e6
-//    232.6 -> 218.2 ms).
+//    under the direction's arithmetic; the Philox key is a kernel argument
+//    (Type Ia packet kernel, 1e6 packets 83.4 -> 77.0 ms, 4e6 231.5 -> 209.4
+//    ms; with eps_imc applied once per zone visit, behind a load at its flush,
+//    4e6 took 216 ms and the grey lightbulb, whose segments end at walls and
+//    bin edges, 1.48 ms instead of 1.37).
 //  * 64 registers, 32 warps per SM: the zone-visit tally sums and the state
 //    a packet reads only at its start or end sit in each thread's slots of
 //    shared memory, and a visit's sums go to one of 32 global tally copies
@@ -131,15 +132,6 @@ __device__ __forceinline__ int next_zone(const StepArgs& A, const GridDev& G, co
   }
   *l = (in_nbr == -1) ? l_in * inv_tiny_offset : l_in * tiny_offset;
   return in_nbr;
-}
-
-// {abs, scat} of bin k of zone iz, from the packed bins {CDF below, CDF, abs,
-// scat} where the context has them
-__device__ __forceinline__ float2 bin_opacity_pair(const StepArgs& A, int iz, int k)
-{
-  const size_t i = (size_t)iz * A.nu.n + k;
-  if (A.bin4) return __ldg(reinterpret_cast<const float2*>(A.bin4 + i) + 1);
-  return __ldg(reinterpret_cast<const float2*>(A.opac) + i);
 }
 
 // a sampled bin: its index, the CDF below and at it, its walls and {abs, scat}
@@ -299,7 +291,7 @@ __device__ __forceinline__ int scatter_batch(const StepArgs& A, Pkt& p, double r
   return kbin;
 }
 
-// adds one zone visit's tallies (the e_abs sum times the zone's eps_imc): to the block's shared copy [5][nz] when
+// adds one zone visit's tallies: to the block's shared copy [5][nz] when
 // A.smem_zones, else to global copy rep_off / (5 nz) of the n_rep copies
 // (rep_off < 0: the arrays themselves).  The targets are formed here, from
 // the shared array and the kernel's arguments, rather than held as five
@@ -488,7 +480,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
   __shared__ int s_oz[SLOTS == 2 ? THREADS : 1];
   auto flush_slot = [&](int z, int k) {  // send slot k's sums for zone z and zero the slot
     double* a = &s_acc[k][0][tid];
-    add_visit(A, s_tal, nz, rep_off, z, a[0] * __ldg(A.eps_imc + z), a[THREADS], a[2 * THREADS], a[3 * THREADS], a[4 * THREADS]);
+    add_visit(A, s_tal, nz, rep_off, z, a[0], a[THREADS], a[2 * THREADS], a[3 * THREADS], a[4 * THREADS]);
     a[0] = 0.0; a[THREADS] = 0.0; a[2 * THREADS] = 0.0; a[3 * THREADS] = 0.0; a[4 * THREADS] = 0.0;
   };
   for (int k = 0; k < SLOTS; ++k)
@@ -667,14 +659,11 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
       nxt_bin = -1;
     } else {
       i_nu = loc_within_mixed(A.nu, p.nu * dshift);
-      if constexpr (BATCH) {
-        ab = __ldg(opac + (size_t)iz * nn + i_nu);
-        dnu_num = (float)(loc_delta(A.nu, i_nu) * A.ct);
-      } else {
-        ab = bin_opacity_pair(A, iz, i_nu);
-        const double2 w = __ldg(A.nu_lr + i_nu);
-        dnu_num = (float)((w.y - w.x) * A.ct);
-      }
+      // from the separate tables: the next bin's pair and walls mostly lie in
+      // the sector just read (from the packed bins, half as many to a sector, the
+      // grey lightbulb, whose segments end at bin edges, ran 1.48 against 1.31 ms)
+      ab = __ldg(opac + (size_t)iz * nn + i_nu);
+      dnu_num = (float)(loc_delta(A.nu, i_nu) * A.ct);
     }
     const float a_f = ab.x;
     const float s_f = A.omit_scat ? 0.0f : ab.y;
@@ -695,12 +684,10 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
     else { event = 2; this_d = d_tm; }
     // tallies (transport.cpp:361-392)
     const double this_E = p.e * this_d;
-    double eps_imc = 1.0;
-    if constexpr (BATCH) eps_imc = __ldg(A.eps_imc + iz);
+    const double eps_imc = __ldg(A.eps_imc + iz);
     const double ed = this_E * dshift;
     double* sa = &s_acc[SLOTS == 2 ? (acc & 1) : 0][0][tid];
-    if constexpr (BATCH) sa[0] = fma(ed * dshift * (double)a_f, eps_imc, sa[0]);
-    else sa[0] = fma(ed * dshift, (double)a_f, sa[0]);  // times eps_imc at the flush: no load per segment
+    sa[0] = fma(ed * dshift * (double)a_f, eps_imc, sa[0]);
     atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
     if (A.tally_forces) {
       const double wd = ed * (double)op_f * dshift;
@@ -741,7 +728,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
         v = __fdividef(num, a_f);
         redist = true;
         if (!A.radiative_eq) {
-          const float ei = (float)(BATCH ? eps_imc : __ldg(A.eps_imc + iz));
+          const float ei = (float)eps_imc;
           if (v > ei) v = __fdividef(v - ei, 1.0f - ei);  // effective scattering
           else { fate = ABSORBED; redist = false; }
         }
