@@ -156,6 +156,22 @@ StepArgs sed::make_step_args(sed_ctx* c, double dt, int64_t n_emit)
   return A;
 }
 
+// The 1D packet kernels of homologous grids add each zone visit's tallies to
+// one of n_rep global copies (block b to copy b % n_rep, fire-and-forget
+// reductions), which the finish kernel sums: against per-block shared-memory
+// copies, whose atomic adds hold the warp, the Type Ia packet kernel ran 563
+// ms against 587 ms (mixed form, 1e7 packets), the FP64 kernel 85 against 89
+// ms (3e5 packets), the grey lightbulb's 26.8 against 28.2 ms.
+int sed::zone_tally_copies(sed_ctx* c, StepArgs& A)
+{
+  const size_t nz = (size_t)c->nz;
+  const int n_rep = (int)std::min<size_t>(32, std::max<size_t>(1, (size_t(256) << 20) / (5 * sizeof(double) * nz)));
+  CK(c->d_zone_rep.resize((size_t)n_rep * 5 * nz));
+  CK(cudaMemsetAsync(c->d_zone_rep.p, 0, (size_t)n_rep * 5 * nz * sizeof(double), c->stream));
+  A.smem_zones = 0; A.n_rep = n_rep; A.zone_rep = c->d_zone_rep.p;
+  return SED_OK;
+}
+
 GridDev sed::make_grid_dev(sed_ctx* c)
 {
   GridDev G{};
@@ -798,15 +814,8 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
     A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_tau = c->d_em_tau.p; A.em_n = n_emit;
   }
   if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G))) {
-    // the 1D packet kernels of homologous grids add each zone visit's tallies to one of n_rep
-    // global copies (block b to copy b % n_rep, fire-and-forget reductions),
-    // which the finish kernel sums: against the per-block shared-memory
-    // copies, whose atomic adds hold the warp, the Type Ia packet kernel ran
-    // 563 ms against 587 ms
-    const int n_rep = (int)std::min<size_t>(32, std::max<size_t>(1, (size_t(256) << 20) / (5 * sizeof(double) * nz)));
-    CK(c->d_zone_rep.resize((size_t)n_rep * 5 * nz));
-    CK(cudaMemsetAsync(c->d_zone_rep.p, 0, (size_t)n_rep * 5 * nz * sizeof(double), c->stream));
-    A.smem_zones = 0; A.n_rep = n_rep; A.zone_rep = c->d_zone_rep.p;
+    const int rc_rep = zone_tally_copies(c, A);
+    if (rc_rep) return rc_rep;
   }
   CK(cudaEventRecord(c->ev[3], c->stream));
   if (A.n_packets > 0) launches += launch_propagate(A, G, c->num_sms, c->stream);
@@ -1138,7 +1147,7 @@ void sed_ctx_destroy(sed_ctx* c)
   DevBuf<int32_t>* ints[] = {&c->d_eZ, &c->d_eA, &c->d_zero_eps_atom, &c->d_ion_off, &c->d_lev_off, &c->d_lev_ion,
                              &c->d_lev_g, &c->d_lev_ic, &c->d_photo_off, &c->d_ion_atom, &c->d_ln_seg,
                              &c->d_fz_seg, &c->d_lev_atom, &c->d_ln_order, &c->d_fz_order, &c->d_solve_err, &c->d_rec_fate, &c->d_rec_ind, &c->d_rec_draws,
-                             &c->d_esc_bin};
+                             &c->d_esc_bin, &c->d_esc_seg, &c->d_replay_order, &c->d_replay_cursor};
   for (auto* b : ints) b->release();
   c->d_ln_lv.release(); c->d_ln_c.release(); c->d_ln_c32.release(); c->d_fz_ia.release(); c->d_fz_c.release();
   c->d_fz_c32.release();

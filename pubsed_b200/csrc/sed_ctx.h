@@ -166,7 +166,9 @@ struct sed_ctx {
   int diff_bands = 0;
   bool diff_scaled = false;
   int64_t diff_n = 0;
-  DevBuf<int32_t> d_esc_bin;
+  DevBuf<int32_t> d_esc_bin, d_esc_seg;
+  DevBuf<int32_t> d_replay_order, d_replay_cursor;  // launch_replay_order
+  bool replay_ordered = false;                      // they belong to the last forward
   DevBuf<double> d_esc_e, d_abs_scale, d_adj_g, d_adj_out;
 
   // per-packet records (also the end states a time-dependent step builds
@@ -257,6 +259,8 @@ int enqueue_opacity(sed_ctx* c, double dt);
 // kernel arguments and device grid of a transport step of this context
 // the packed bins again, after the {abs, scat} or CDF tables were written by something else than an opacity build
 cudaError_t pack_bins(sed_ctx* c);
+// the zone-scalar tallies of a step in copies (zeroed), for the packet and finish kernels
+int zone_tally_copies(sed_ctx* c, StepArgs& A);
 StepArgs make_step_args(sed_ctx* c, double dt, int64_t n_emit);
 GridDev make_grid_dev(sed_ctx* c);
 

@@ -10,6 +10,7 @@
 // segment and +w per scattering (the score of the scattering path, a
 // likelihood-ratio term, since the scattering opacity decides where the
 // path goes).  Nothing of a path is stored between the two launches.
+#include <cstdint>
 #include <cstring>
 #include <vector>
 
@@ -69,6 +70,19 @@ int replay(sed_ctx* c, bool jacobian, sed_step_stats* st, bool density = false)
   A.adj_density = density ? 1 : 0;
   CK(cudaMemsetAsync(c->d_counters.p, 0, (C_COUNT + 1) * sizeof(unsigned long long), c->stream));
   CK(cudaEventRecord(c->ev[3], c->stream));
+  int launches = c->diff_n > 0 ? 1 : 0;
+  if (c->tp.precision && c->diff_n > 0 && c->diff_n <= INT32_MAX) {
+    if (!c->replay_ordered) {
+      CK(c->d_replay_order.resize((size_t)c->diff_n));
+      CK(c->d_replay_cursor.resize(REPLAY_BUCKETS + 1));
+      launches += launch_replay_order(c->d_esc_bin.p, c->d_esc_seg.p, c->diff_n, c->d_replay_order.p,
+                                      c->d_replay_cursor.p, c->num_sms, c->stream);
+      CK(cudaGetLastError());
+      c->replay_ordered = true;
+    }
+    A.replay_order = c->d_replay_order.p;
+    A.n_replay = c->d_replay_cursor.p + REPLAY_BUCKETS;
+  }
   if (c->diff_n > 0 && launch_propagate_diff(A, make_grid_dev(c), 2, c->num_sms, c->stream) < 0)
     return set_err(c, SED_ERR_ARG, "adjoint replay: unsupported grid");
   CK(cudaGetLastError());
@@ -78,7 +92,7 @@ int replay(sed_ctx* c, bool jacobian, sed_step_stats* st, bool density = false)
   CK(cudaStreamSynchronize(c->stream));
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev[3], c->ev[4]);
-  fill_stats(st, cnt, c->diff_n, ms, ms, c->diff_n > 0 ? 1 : 0);
+  fill_stats(st, cnt, c->diff_n, ms, ms, launches);
   if (cnt[C_LIMIT] > 0) return set_err(c, SED_ERR_LIMIT, "%llu packets hit the segment limit", cnt[C_LIMIT]);
   return SED_OK;
 }
@@ -129,6 +143,8 @@ int diff_forward(sed_ctx* c, double dt, const double* abs_scale, cudaMemcpyKind 
   const size_t nz = (size_t)c->nz, nn = (size_t)c->nu.n(), nj = c->tp.store_Jnu ? nn : 1;
   CK(c->d_esc_bin.resize((size_t)std::max<int64_t>(n_emit, 1)));
   CK(c->d_esc_e.resize((size_t)std::max<int64_t>(n_emit, 1)));
+  if (c->tp.precision) CK(c->d_esc_seg.resize((size_t)std::max<int64_t>(n_emit, 1)));
+  c->replay_ordered = false;
   if (abs_scale) {
     CK(c->d_abs_scale.resize(nz * (size_t)n_bands));
     CK(cudaMemcpyAsync(c->d_abs_scale.p, abs_scale, nz * (size_t)n_bands * sizeof(double), in, c->stream));
@@ -152,10 +168,16 @@ int diff_forward(sed_ctx* c, double dt, const double* abs_scale, cudaMemcpyKind 
   A.abs_scale = abs_scale ? c->d_abs_scale.p : nullptr;
   A.esc_bin = c->d_esc_bin.p;
   A.esc_e = c->d_esc_e.p;
+  A.esc_seg = c->d_esc_seg.p;
   if (c->record) {
     A.rec_fate = c->d_rec_fate.p; A.rec_ind = c->d_rec_ind.p; A.rec_draws = c->d_rec_draws.p; A.rec_state = c->d_rec_state.p;
   }
   const GridDev G = make_grid_dev(c);
+  if (c->gtype == SED_GRID_1D_SPHERE && c->tp.precision) {
+    // zone-scalar tallies in copies, as for the 1D packet kernels of a plain step
+    const int rc_rep = zone_tally_copies(c, A);
+    if (rc_rep) return rc_rep;
+  }
   int launches = 0;
   CK(cudaEventRecord(c->ev[3], c->stream));
   if (n_emit > 0) {

@@ -97,6 +97,9 @@ struct StepArgs {
   int32_t adj_density;               // adjoint: 1 = d / d ln rho per zone (likelihood-ratio score + absorption)
   int32_t* esc_bin;                  // [n_packets] spectrum index of an escaped, counted packet; -1 otherwise
   double* esc_e;                     // [n_packets] its energy at escape
+  int32_t* esc_seg;                  // [n_packets] its segments (FP32-table kernels)
+  const int32_t* replay_order;       // [n_replay] the packets a replay walks, longest first; or null: all of them
+  const int32_t* n_replay;           // device scalar
   const double* adj_g;               // [nspec] d(loss)/d(flux) for the vector-Jacobian product
   double* adj_out;                   // VJP [nz * n_bands]; Jacobian [nspec * nz * n_bands]
 };
@@ -211,6 +214,11 @@ int launch_finish(const StepArgs& a, const GridDev& g, const double* vol, int64_
 // a continuous weight (interactions sampled from scattering only), mode 2 =
 // adjoint replay of the escaped packets of the last mode-1 launch.
 int launch_propagate_diff(const StepArgs& a, const GridDev& g, int mode, int num_sms, cudaStream_t s);
+// the escaped packets of a weighted forward by decreasing segment count, into
+// order[n]; cursor: [REPLAY_BUCKETS + 1] scratch whose last entry becomes their number
+constexpr int REPLAY_BUCKETS = 2048;
+int launch_replay_order(const int32_t* esc_bin, const int32_t* esc_seg, int64_t n, int32_t* order, int32_t* cursor,
+                        int num_sms, cudaStream_t s);
 
 // Batched packet kernel: compiled shapes {threads per block, min blocks per
 // SM} selectable at run time (the autotuner times each).  `blocks_per_sm`

@@ -1888,6 +1888,7 @@ __global__ void init_particles_kernel(const InitArgs I, const GridDev G)
 
 #include "mixed_kernel.cuh"
 #include "fp64_kernel.cuh"
+#include "diff_kernel.cuh"
 
 // Blocks of a persistent packet kernel, `per_sm` of which fit on an SM, and
 // the lanes of a warp that take packets.  With fewer packets than the chip has
@@ -2092,15 +2093,36 @@ int launch_finish(const StepArgs& a, const GridDev& g, const double* vol, int64_
   return n + 1;
 }
 
-template <int GRID>
-int launch_diff_t(const StepArgs& b, const GridDev& g, int mode, int num_sms, cudaStream_t s)
+// differentiable transport on FP32 tables: the forward at 28 warps per SM, the
+// replay, whose warps hold packets of one length, at 20 (1e6 Type Ia packets,
+// 16 / 20 / 24 / 28 / 32 warps: forward 85.7 / 89.5 / 91.5 / 86.4 / 93.9 ms,
+// replay 56.8 / 55.7 / 61.2 / 62.3 / 70.1 ms)
+template <int GRID, int MODE>
+int launch_diff_t(const StepArgs& b, const GridDev& g, int num_sms, cudaStream_t s)
 {
   constexpr int T = SED_PROP_THREADS, B = SED_PROP_MINB;
-  if (b.precision == 0)
-    return mode == 1 ? launch_kernel_t<GRID, double2, double, 0, T, B, 1>(b, g, 0, num_sms, b.n_packets, s)
-                     : launch_kernel_t<GRID, double2, double, 0, T, B, 2>(b, g, 0, num_sms, b.n_packets, s);
-  return mode == 1 ? launch_kernel_t<GRID, float2, float, 0, T, B, 1>(b, g, 0, num_sms, b.n_packets, s)
-                   : launch_kernel_t<GRID, float2, float, 0, T, B, 2>(b, g, 0, num_sms, b.n_packets, s);
+  if (b.precision == 0) return launch_kernel_t<GRID, double2, double, 0, T, B, MODE>(b, g, 0, num_sms, b.n_packets, s);
+  constexpr int DT = 128;
+  auto kern = propagate_diff_kernel<GRID, MODE, DT, (MODE == 1 ? 7 : 5)>;
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DT, 0);
+  if (per_sm < 1) per_sm = 1;
+  StepArgs a = b;
+  a.smem_zones = 0;
+  const int64_t blocks = spread_packets(a.n_packets, DT, per_sm, num_sms, &a.lanes);
+  kern<<<(unsigned)blocks, DT, 0, s>>>(a, g);
+  return 1;
+}
+
+int launch_replay_order(const int32_t* esc_bin, const int32_t* esc_seg, int64_t n, int32_t* order, int32_t* cursor,
+                        int num_sms, cudaStream_t s)
+{
+  const unsigned b = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)num_sms * 8, (n + 255) / 256));
+  cudaMemsetAsync(cursor, 0, (REPLAY_BUCKETS + 1) * sizeof(int32_t), s);
+  replay_count_kernel<<<b, 256, 0, s>>>(esc_bin, esc_seg, n, cursor);
+  replay_scan_kernel<<<1, 1024, 0, s>>>(cursor);
+  replay_place_kernel<<<b, 256, 0, s>>>(esc_bin, esc_seg, n, cursor, order);
+  return 3;
 }
 
 int launch_propagate_diff(const StepArgs& a, const GridDev& g, int mode, int num_sms, cudaStream_t s)
@@ -2108,7 +2130,8 @@ int launch_propagate_diff(const StepArgs& a, const GridDev& g, int mode, int num
   if (!g.homologous || (mode != 1 && mode != 2)) return -1;
   StepArgs b = a;
   if (mode == 2) b.smem_zones = 0;  // the replay tallies nothing per zone
-  return g.type == 0 ? launch_diff_t<0>(b, g, mode, num_sms, s) : launch_diff_t<1>(b, g, mode, num_sms, s);
+  if (mode == 1) return g.type == 0 ? launch_diff_t<0, 1>(b, g, num_sms, s) : launch_diff_t<1, 1>(b, g, num_sms, s);
+  return g.type == 0 ? launch_diff_t<0, 2>(b, g, num_sms, s) : launch_diff_t<1, 2>(b, g, num_sms, s);
 }
 
 int launch_gamma(const StepArgs& a, const StepArgs& ag, const RadioArgs& r, const GridDev& g, int num_sms,
