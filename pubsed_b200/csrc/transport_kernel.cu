@@ -965,6 +965,8 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
   }
 }
 
+constexpr int FINISH_THREADS = 256, FINISH_BATCH = 8;
+
 // reduce_radiation normalisation (src/transport/transport_mpi.cpp:415-441)
 // of zone iz, after the steady-state luminosity rescale (transport.cpp:94-115)
 // by `fac` when do_rescale.  Run by one block per zone.
@@ -974,24 +976,37 @@ __device__ __forceinline__ void finish_zone(const StepArgs& A, const double* __r
   const int nn = A.nu.n;
   const double dt = A.dt;
   const double v = vol[iz];
-  __shared__ double red[256];
+  __shared__ double red[8];
   if (A.store_Jnu && nn > 1) {
     double* J = A.J + (size_t)iz * nn;
+    const double den = v * dt * 4 * PI;
     double esum = 0;
-    for (int j = threadIdx.x; j < nn; j += blockDim.x) {
-      double x = J[j];
-      if (do_rescale) x *= fac;
-      const double d = loc_delta(A.nu, j);
-      x /= v * dt * 4 * PI * d;
-      J[j] = x;
-      esum += x * d * 4 * PI / C_LIGHT;
+    // FINISH_BATCH bins of a thread are in flight together: a load, a division
+    // and a store per turn waited for DRAM once per bin
+    for (int j0 = threadIdx.x; j0 < nn; j0 += FINISH_BATCH * FINISH_THREADS) {
+      double x[FINISH_BATCH];
+#pragma unroll
+      for (int k = 0; k < FINISH_BATCH; ++k) {
+        const int j = j0 + k * FINISH_THREADS;
+        x[k] = (j < nn) ? __ldcs(J + j) : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < FINISH_BATCH; ++k) {
+        const int j = j0 + k * FINISH_THREADS;
+        if (j < nn) {
+          const double d = loc_delta(A.nu, j);
+          double y = x[k];
+          if (do_rescale) y *= fac;
+          y /= den * d;
+          __stcs(J + j, y);
+          esum += y * d;
+        }
+      }
     }
-    red[threadIdx.x] = esum;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) esum += __shfl_xor_sync(0xffffffffu, esum, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = esum;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < (unsigned)s) red[threadIdx.x] += red[threadIdx.x + s];
-      __syncthreads();
-    }
   }
   if (threadIdx.x == 0) {
     A.e_abs[iz] /= v * dt;
@@ -1005,7 +1020,9 @@ __device__ __forceinline__ void finish_zone(const StepArgs& A, const double* __r
       if (do_rescale && A.store_Jnu) { j0 *= fac; A.J[(size_t)iz * nn] = j0; }
       A.e_rad[iz] = j0 / (v * dt * C_LIGHT);
     } else {
-      A.e_rad[iz] = red[0];
+      double sum = 0;
+      for (int w = 0; w < FINISH_THREADS / 32; ++w) sum += red[w];
+      A.e_rad[iz] = sum * 4 * PI / C_LIGHT;
     }
   }
 }
@@ -2089,7 +2106,7 @@ int launch_finish(const StepArgs& a, const GridDev& g, const double* vol, int64_
     rescale_spectrum_kernel<<<64, 256, 0, s>>>(a, nspec, a.n_packets);
     ++n;
   }
-  finish_zones_kernel<<<g.nzones, 256, 0, s>>>(a, vol, g.nzones, a.n_packets, rescale);
+  finish_zones_kernel<<<g.nzones, FINISH_THREADS, 0, s>>>(a, vol, g.nzones, a.n_packets, rescale);
   return n + 1;
 }
 
@@ -2215,7 +2232,7 @@ int launch_finish_batch(const StepArgs& a, const double* vol, int nz_total, int6
     rescale_spectrum_batch_kernel<<<148, 256, 0, s>>>(a, nspec);
     ++n;
   }
-  finish_zones_batch_kernel<<<nz_total, 256, 0, s>>>(a, vol, nz_total, rescale);
+  finish_zones_batch_kernel<<<nz_total, FINISH_THREADS, 0, s>>>(a, vol, nz_total, rescale);
   return n + 1;
 }
 
