@@ -116,10 +116,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_diff_kernel(const Ste
   int ind_in = -1;
   double adj_w = 0, acc_g = 0;  // replay: the packet's weight, the sum of one (zone, band)
   int64_t adj_row = 0, acc_key = -1;
-  auto block = [&](uint32_t n) {
-    const PhiloxOut o = philox4x32_10(n, (uint32_t)stream, (uint32_t)(stream >> 32), A.step, A.seed, 1u);
-    return make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
-  };
+  auto block = [&](uint32_t n) { return philox_words(A, stream, n); };
   auto flush = [&](int z) {
     mixed::add_visit(A, nullptr, nz, rep_off, z, s_acc[0][tid], s_acc[MODE == 1 ? 1 : 0][tid],
                      s_acc[MODE == 1 ? 2 : 0][tid], s_acc[MODE == 1 ? 3 : 0][tid], s_acc[MODE == 1 ? 4 : 0][tid]);

@@ -376,7 +376,8 @@ __device__ __forceinline__ void load_emitted(const StepArgs& A, Pkt& p, int64_t 
 // kernel.  Emission is the longest stretch of the packet kernel's loop
 // (double-precision sincos, searches of the core CDF and of the zone walls);
 // inside the persistent loop one lane emitting holds its whole warp.
-template <int BATCH>
+// GRID 1: a 3D step's core packets, which need no optical depth (em_tau null).
+template <int BATCH, int GRID>
 __global__ void __launch_bounds__(256) emit_mixed_kernel(const StepArgs A, const GridDev G)
 {
   using namespace mixed;
@@ -404,15 +405,15 @@ __global__ void __launch_bounds__(256) emit_mixed_kernel(const StepArgs A, const
     } else {
       rng.init(A.seed, (uint64_t)A.first_pid + q, step, 0);
       DrawWords d{rng};
-      emit_core<0>(A, G, p, d, A.core_radius, A.Ep, A.core_cdf, GridZoneOf<0>{G});
-      tau = neg_log_u(d.word());
+      emit_core<GRID>(A, G, p, d, A.core_radius, A.Ep, A.core_cdf, GridZoneOf<GRID>{G});
+      tau = (GRID == 0) ? neg_log_u(d.word()) : 0.f;
     }
     double* s = A.em_state + q;
     s[0] = p.x[0]; s[n] = p.x[1]; s[2 * n] = p.x[2];
     s[3 * n] = p.D[0]; s[4 * n] = p.D[1]; s[5 * n] = p.D[2];
     s[6 * n] = p.t; s[7 * n] = p.e; s[8 * n] = p.nu;
     A.em_ind[q] = p.ind;
-    A.em_tau[q] = tau;
+    if (GRID == 0) A.em_tau[q] = tau;
   }
 }
 

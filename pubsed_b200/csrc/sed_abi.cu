@@ -148,6 +148,8 @@ StepArgs sed::make_step_args(sed_ctx* c, double dt, int64_t n_emit)
   A.opac = c->d_opac.p; A.cdf = c->d_cdf.p; A.eps_imc = c->d_eps_imc.p;
   A.cdf_coarse = c->d_cdf_coarse.p; A.n_coarse = c->n_coarse;
   A.bin4 = c->d_bin4.p; A.nu_lr = c->d_nu_lr.p;
+  if (c->d_ax_push.p)
+    for (int a = 0, o = 0; a < 3; o += c->ax[a++].n()) A.ax_push[a] = c->d_ax_push.p + o;
   A.cdf_guide = c->guide_n ? c->d_cdf_guide.p : nullptr; A.guide_n = c->guide_n;
   A.rescale_lum = c->tp.core_fix_luminosity;
   A.J = c->d_J.p; A.e_abs = c->d_e_abs.p; A.e_rad = c->d_e_rad.p;
@@ -329,6 +331,9 @@ int sed_set_grid(sed_ctx* c, const sed_grid* g)
       c->ax[a] = host_loc(*axes[a]);
       CK(upload(c, c->d_ax[a], c->ax[a].x.data(), c->ax[a].x.size()));
     }
+    CK(c->d_ax_push.resize((size_t)c->nx + c->ny + c->nzz));
+    for (int a = 0, o = 0; a < 3; o += c->ax[a++].n()) launch_pushed_walls(dev_loc(c->ax[a], c->d_ax[a]), c->d_ax_push.p + o, c->stream);
+    CK(cudaGetLastError());
   } else {
     return set_err(c, SED_ERR_ARG, "sed_set_grid: unknown grid type %d", g->type);
   }
@@ -813,7 +818,18 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
     CK(c->d_em_tau.resize((size_t)n_emit));
     A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_tau = c->d_em_tau.p; A.em_n = n_emit;
   }
-  if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G))) {
+  if (cart_path(A, G) && n_emit > 0 && n_q == 0) {
+    // core packets emitted ahead where the memory holds them (80 B each), in the packet kernel otherwise
+    if (c->d_em_state.resize((size_t)n_emit * 9) == cudaSuccess && c->d_em_ind.resize((size_t)n_emit) == cudaSuccess) {
+      A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_n = n_emit;
+    } else {
+      cudaGetLastError();
+      c->d_em_state.release();
+      c->d_em_ind.release();
+    }
+  }
+  // (on a 3D grid of few cells too, where direct adds would meet on the same addresses)
+  if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G)) || (cart_path(A, G) && nz <= 8192)) {
     const int rc_rep = zone_tally_copies(c, A);
     if (rc_rep) return rc_rep;
   }
@@ -1152,7 +1168,7 @@ void sed_ctx_destroy(sed_ctx* c)
   c->d_ln_lv.release(); c->d_ln_c.release(); c->d_ln_c32.release(); c->d_fz_ia.release(); c->d_fz_c.release();
   c->d_fz_c32.release();
   c->d_opac.release(); c->d_cdf.release(); c->d_cdf_coarse.release(); c->d_counters.release();
-  c->d_cdf_guide.release(); c->d_bin4.release(); c->d_nu_lr.release();
+  c->d_cdf_guide.release(); c->d_bin4.release(); c->d_nu_lr.release(); c->d_ax_push.release();
   c->d_temp_bad.release();
   DevBuf<double>* rad[] = {&c->d_gn, &c->d_gflux, &c->d_gclick, &c->d_radio_cdf, &c->d_gamma_frac, &c->d_compton,
                            &c->d_photoion, &c->d_L_emit, &c->d_L_dep, &c->d_L_tot, &c->d_q_state};

@@ -129,6 +129,7 @@ struct sed_ctx {
   int n_coarse = 0;
   bool in_batch = false;         // the inner context of a batch
   DevBuf<float4> d_bin4;         // packed bins of the 1D mixed packet kernel (FP32 tables on 1D grids)
+  DevBuf<double2> d_ax_push;     // 3D: pushed walls of the three axes, one after the other
   DevBuf<double2> d_nu_lr;       // {left, right} walls of the frequency bins
   DevBuf<uint16_t> d_cdf_guide;  // CDF guide tables, guide_n + 1 entries per zone
   int guide_n = 0;

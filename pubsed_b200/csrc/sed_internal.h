@@ -89,6 +89,7 @@ struct StepArgs {
   int32_t* em_ind;                   // [n] its zone (or -1 / -2)
   float* em_tau;                     // [n] optical depth of its first flight
   int32_t* em_model;                 // [n] its model (batches)
+  const double2* ax_push[3];         // 3D mixed kernel: {left, right} wall of a cell, pushed outwards, per axis
   int64_t em_n;                      // core packets emitted there (the stride of em_state)
   // ---- differentiable transport (weighted forward and adjoint replay kernels only) ----
   const double* abs_scale;           // [nz * n_bands] factor on the absorption opacity, or null
@@ -204,6 +205,11 @@ int launch_propagate(const StepArgs& a, const GridDev& g, int num_sms, cudaStrea
 bool mixed_1d_path(const StepArgs& a, const GridDev& g);
 // whether it runs the FP64 kernel of homologous grids (fp64_kernel.cuh)
 bool fp64_path(const StepArgs& a, const GridDev& g);
+// whether it runs the 3D mixed kernel (cart_kernel.cuh): with em_n core packets
+// emitted ahead when they are all the step has and the em_* buffers are given
+bool cart_path(const StepArgs& a, const GridDev& g);
+// the pushed walls of an axis for it
+int launch_pushed_walls(const DevLoc& ax, double2* out, cudaStream_t s);
 // IMD probabilities of the step (transport::compute_diffusion_probabilities)
 // from the zone Planck means into out[4][nz]
 int launch_imd_probabilities(const GridDev& g, const double* planck, double dt, double* out, cudaStream_t s);

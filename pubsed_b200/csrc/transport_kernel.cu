@@ -1903,9 +1903,18 @@ __global__ void init_particles_kernel(const InitArgs I, const GridDev G)
   }
 }
 
+// block n of a stream in the word layout (PacketRng::block), with the step's
+// key and number, the kernel's arguments
+__device__ __forceinline__ uint4 philox_words(const StepArgs& A, uint64_t stream, uint32_t n)
+{
+  const PhiloxOut o = philox4x32_10(n, (uint32_t)stream, (uint32_t)(stream >> 32), A.step, A.seed, 1u);
+  return make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
+}
+
 #include "mixed_kernel.cuh"
 #include "fp64_kernel.cuh"
 #include "diff_kernel.cuh"
+#include "cart_kernel.cuh"
 
 // Blocks of a persistent packet kernel, `per_sm` of which fit on an SM, and
 // the lanes of a warp that take packets.  With fewer packets than the chip has
@@ -1946,7 +1955,7 @@ int launch_mixed_t(const StepArgs& a0, const GridDev& g, int blocks_per_sm, int 
   if (a.em_n > 0) {  // the core packets, emitted ahead
     int64_t eb = (a.em_n + 255) / 256;
     if (eb > (int64_t)num_sms * 16) eb = (int64_t)num_sms * 16;
-    emit_mixed_kernel<BATCH><<<(unsigned)eb, 256, 0, s>>>(a, g);
+    emit_mixed_kernel<BATCH, 0><<<(unsigned)eb, 256, 0, s>>>(a, g);
   }
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
@@ -2005,6 +2014,28 @@ bool fp64_ok(const StepArgs& a, const GridDev& g)
   return a.precision == 0 && g.homologous && a.use_ddmc == 0 && a.t_grid > 1e-100 && a.t_grid < 1e100;
 }
 
+// The 3D mixed form: 28 warps per SM at 72 registers, no spills (2e6 packets,
+// packet kernel, 40^3 / 64^3 cells: propagate_kernel at the same shape 41.8 /
+// 59.7 ms; here 24, 28, 32, 36 warps 30.5 / 49.1, 29.9 / 48.5, 30.7 / 49.1, 31.7 /
+// 50.3 ms).
+int launch_cart(const StepArgs& a0, const GridDev& g, int num_sms, cudaStream_t s)
+{
+  constexpr int T = 128, B = 7;
+  StepArgs a = a0;
+  a.smem_zones = 0;
+  const bool ahead = a.em_n > 0;
+  auto kern = ahead ? propagate_cart_kernel<0, T, B> : propagate_cart_kernel<1, T, B>;
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, 0);
+  if (per_sm < 1) per_sm = 1;
+  const int64_t blocks = spread_packets(a.n_packets, T, per_sm, num_sms, &a.lanes);
+  const unsigned eb = (unsigned)std::min<int64_t>((a.em_n + 255) / 256, (int64_t)num_sms * 16);
+  if (ahead) emit_mixed_kernel<0, 1><<<eb, 256, 0, s>>>(a, g);
+  kern<<<(unsigned)blocks, T, 0, s>>>(a, g);
+  if (ahead) count_escaped_kernel<<<eb, 256, 0, s>>>(a);
+  return ahead ? 3 : 1;
+}
+
 template <int GRID, typename OT, typename CT>
 int launch_propagate_t(const StepArgs& a, const GridDev& g, int num_sms, cudaStream_t s)
 {
@@ -2019,7 +2050,7 @@ int launch_propagate_t(const StepArgs& a, const GridDev& g, int num_sms, cudaStr
     return launch_kernel_t<GRID, OT, CT, 0, 256, 4, 0, false>(a, g, 0, num_sms, a.n_packets, s);
   if constexpr (sizeof(OT) == sizeof(float2)) {
     if constexpr (GRID == 0) return launch_mixed_t<0, SED_MIXED_THREADS, SED_MIXED_MINB>(a, g, 0, num_sms, a.n_packets, s);
-    else return launch_kernel_t<GRID, OT, CT, 0, 128, 7>(a, g, 0, num_sms, a.n_packets, s);
+    else return launch_cart(a, g, num_sms, s);
   } else {
     if (fp64_ok(a, g)) {
       // few packets wait for the longest chain: 16 warps per SM at 112
@@ -2090,6 +2121,17 @@ int launch_propagate(const StepArgs& a, const GridDev& g, int num_sms, cudaStrea
   }
   if (a.precision == 0) return launch_propagate_t<1, double2, double>(a, g, num_sms, s);
   return launch_propagate_t<1, float2, float>(a, g, num_sms, s);
+}
+
+bool cart_path(const StepArgs& a, const GridDev& g)
+{
+  return a.precision != 0 && g.type == 1 && g.homologous && a.use_ddmc == 0;
+}
+
+int launch_pushed_walls(const DevLoc& ax, double2* out, cudaStream_t s)
+{
+  pushed_walls_kernel<<<(ax.n + 127) / 128, 128, 0, s>>>(ax, out);
+  return 1;
 }
 
 int launch_imd_probabilities(const GridDev& g, const double* planck, double dt, double* out, cudaStream_t s)
