@@ -177,7 +177,8 @@ int sed::zone_tally_copies(sed_ctx* c, StepArgs& A)
 GridDev sed::make_grid_dev(sed_ctx* c)
 {
   GridDev G{};
-  G.type = c->gtype; G.nzones = c->nz; G.homologous = c->homologous; G.t_grid = c->t_grid;
+  G.type = c->gtype; G.nzones = c->nz; G.homologous = c->homologous;
+  set_grid_time(G, c->t_grid);
   if (c->gtype == SED_GRID_1D_SPHERE) {
     G.r_out = dev_loc(c->r_out, c->d_r_out);
     G.v_r = c->d_v_r.p;

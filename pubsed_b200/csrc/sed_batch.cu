@@ -163,7 +163,8 @@ GridDev grid_dev(sed_batch* b)
 {
   sed_ctx* c = b->inner;
   GridDev G{};
-  G.type = SED_GRID_1D_SPHERE; G.nzones = c->nz; G.homologous = 1; G.t_grid = c->t_grid;
+  G.type = SED_GRID_1D_SPHERE; G.nzones = c->nz; G.homologous = 1;
+  set_grid_time(G, c->t_grid);
   G.r_out = dev_loc(c->r_out, c->d_r_out);
   G.v_r = nullptr;
   return G;

@@ -14,6 +14,7 @@ struct GridDev {
   int32_t homologous;
   int32_t nx, ny, nz;
   double t_grid;      // homologous velocity v = x / t_grid
+  double inv_t, inv_t_lo;  // 1/t_grid and what its rounding left; 0: t_grid outside what div_by takes
   DevLoc r_out;       // 1D: zone right walls (flex), min = r_min
   const double* v_r;  // 1D non-homologous zone velocities
   DevLoc ax[3];       // 3D axes
@@ -197,6 +198,7 @@ struct BatchModel {
 
 // the grid-time factors of a step's arguments: 1/t, c t and their like
 void set_grid_time(StepArgs& a, double t_grid);
+void set_grid_time(GridDev& g, double t_grid);
 // launches the persistent packet kernel; returns the number of launches
 int launch_propagate(const StepArgs& a, const GridDev& g, int num_sms, cudaStream_t s);
 // whether launch_propagate runs the mixed-form 1D kernel for these

@@ -62,7 +62,7 @@ __device__ __forceinline__ int get_next_zone(const GridDev& G, const double* x, 
 {
   if constexpr (GRID == 0) {
     const double r_o = __ldg(G.r_out.right + i);
-    const double l_out = -1 * xdotD + sqrt(xdotD * xdotD + r_o * r_o - rsq);
+    const double l_out = -1 * xdotD + sqrt_rn(xdotD * xdotD + r_o * r_o - rsq);
     double r_in;
     int ind_in;
     if (i != 0) { r_in = __ldg(G.r_out.right + i - 1); ind_in = i - 1; }
@@ -118,6 +118,12 @@ __device__ __forceinline__ void get_velocity(const GridDev& G, int i, const doub
                                              double* dvds)
 {
   if (G.homologous) {
+    if (G.inv_t != 0) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = div_by(x[k], G.t_grid, G.inv_t, G.inv_t_lo);
+      *dvds = G.inv_t;
+      return;
+    }
     v[0] = x[0] / G.t_grid;
     v[1] = x[1] / G.t_grid;
     v[2] = x[2] / G.t_grid;
@@ -129,23 +135,39 @@ __device__ __forceinline__ void get_velocity(const GridDev& G, int i, const doub
     // the grid (discrete_diffusion.cpp:324-328), where the reference reads
     // past its zone array; the last zone's velocity field is used instead
     if (i >= G.nzones) i = G.nzones - 1;
-    const double rr = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+    const double rr = sqrt_rn(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
     double v_0, r_0;
     if (i == 0) { v_0 = 0; r_0 = G.r_out.min; }
     else { v_0 = __ldg(G.v_r + i - 1); r_0 = __ldg(G.r_out.right + i - 1); }
     const double dr = rr - r_0;
-    const double dv_dr = (__ldg(G.v_r + i) - v_0) / (__ldg(G.r_out.right + i) - r_0);
+    const double dv_dr = div_rn(__ldg(G.v_r + i) - v_0, __ldg(G.r_out.right + i) - r_0);
     const double vv = v_0 + dv_dr * dr;
-    const double Ddr = (D[0] * x[0] + D[1] * x[1] + D[2] * x[2]) / rr;
-    v[0] = x[0] / rr * vv;
-    v[1] = x[1] / rr * vv;
-    v[2] = x[2] / rr * vv;
-    *dvds = Ddr * Ddr * (dv_dr - vv / rr) + vv / rr;
+    const double y = rcp_rn(rr), v_rr = div_rn(vv, rr, y);
+    const double Ddr = div_rn(D[0] * x[0] + D[1] * x[1] + D[2] * x[2], rr, y);
+    v[0] = div_rn(x[0], rr, y) * vv;
+    v[1] = div_rn(x[1], rr, y) * vv;
+    v[2] = div_rn(x[2], rr, y) * vv;
+    *dvds = Ddr * Ddr * (dv_dr - v_rr) + v_rr;
     if (rr == 0) { v[0] = v[1] = v[2] = 0; *dvds = dv_dr; }
   } else {
     v[0] = v[1] = v[2] = 0;
     *dvds = 0;
   }
+}
+
+// The general kernel and the helpers below divide and take roots with
+// rcp_rn, div_rn and sqrt_rn: a packet is one serial chain, and CUDA's own
+// division (114 cycles here, one after the other since each ends in a branch)
+// was most of it.  The quotients are the same bits, shared divisors share one
+// reciprocal, and independent ones overlap.  Outside the normal range, where
+// opacities can lie, the plain operators answer.
+// (Gaussian pulse with discrete diffusion, 1e6 packets, eight steps of the
+// kernel: 133 -> 125 ms.)
+__device__ __forceinline__ double rcp_any(double b) { return (b > 1e-290 && b < 1e290) ? rcp_rn(b) : 1.0 / b; }
+__device__ __forceinline__ double absorbed_part(double a_opac, double op)
+{
+  if (op > 1e-290 && op < 1e290) return div_rn(a_opac, op);
+  return (op == 0) ? 0 : a_opac / op;
 }
 
 // transport::do_dshift lab -> comoving (src/transport/relativity.cpp:14-43)
@@ -154,11 +176,11 @@ __device__ __forceinline__ double dshift_lab_to_comoving(const GridDev& G, Pkt& 
 {
   double v[3], dvds;
   get_velocity<GRID>(G, p.ind, p.x, p.D, v, &dvds);
-  const double beta2 = (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) / C_LIGHT / C_LIGHT;
+  const double beta2 = div_c(div_c(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
   const double vdd = v[0] * p.D[0] + v[1] * p.D[1] + v[2] * p.D[2];
-  const double gamma = 1.0 / sqrt(1 - beta2);
+  const double gamma = rcp_sqrt_rn(1 - beta2);
   p.dvds = dvds;
-  return gamma * (1 - vdd / C_LIGHT);
+  return gamma * (1 - div_c(vdd));
 }
 
 // transport::lorentz_transform(p, 1) (relativity.cpp:84-127)
@@ -168,21 +190,21 @@ __device__ __forceinline__ void comoving_to_lab(const GridDev& G, Pkt& p)
   double v[3], dvds;
   get_velocity<GRID>(G, p.ind, p.x, p.D, v, &dvds);
   v[0] *= -1; v[1] *= -1; v[2] *= -1;
-  const double beta2 = (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) / C_LIGHT / C_LIGHT;
+  const double beta2 = div_c(div_c(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
   const double vdd = v[0] * p.D[0] + v[1] * p.D[1] + v[2] * p.D[2];
-  const double gamma = 1.0 / sqrt(1 - beta2);
-  const double dshift = gamma * (1 - vdd / C_LIGHT);
+  const double gamma = rcp_sqrt_rn(1 - beta2);
+  const double dshift = gamma * (1 - div_c(vdd));
   p.dvds = dvds;
   p.e *= dshift;
   p.nu *= dshift;
-  const double f = (1 - gamma * vdd / C_LIGHT / (gamma + 1));
-  p.D[0] = 1.0 / dshift * (p.D[0] - gamma * v[0] / C_LIGHT * f);
-  p.D[1] = 1.0 / dshift * (p.D[1] - gamma * v[1] / C_LIGHT * f);
-  p.D[2] = 1.0 / dshift * (p.D[2] - gamma * v[2] / C_LIGHT * f);
+  const double f = (1 - div_rn(div_c(gamma * vdd), gamma + 1));
+  const double inv = rcp_rn(dshift);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p.D[k] = inv * (p.D[k] - div_c(gamma * v[k]) * f);
   const double norm = p.D[0] * p.D[0] + p.D[1] * p.D[1] + p.D[2] * p.D[2];
-  p.D[0] /= norm;
-  p.D[1] /= norm;
-  p.D[2] /= norm;
+  const double y = rcp_rn(norm);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p.D[k] = div_rn(p.D[k], norm, y);
 }
 
 // ----------------------------------------------------------- batches
@@ -278,9 +300,9 @@ __device__ __forceinline__ void isotropic_scatter(const StepArgs& A, const GridD
   double V[3], dvds;
   get_velocity<GRID>(G, p.ind, p.x, p.D, V, &dvds);
   const double vdotD = V[0] * p.D[0] + V[1] * p.D[1] + V[2] * p.D[2];
-  const double beta2 = (V[0] * V[0] + V[1] * V[1] + V[2] * V[2]) / C_LIGHT / C_LIGHT;
-  const double gamma = 1.0 / sqrt(1 - beta2);
-  const double dshift_in = gamma * (1 - vdotD / C_LIGHT);
+  const double beta2 = div_c(div_c(V[0] * V[0] + V[1] * V[1] + V[2] * V[2]));
+  const double gamma = rcp_sqrt_rn(1 - beta2);
+  const double dshift_in = gamma * (1 - div_c(vdotD));
   p.e = p.e * dshift_in;
   p.nu = p.nu * dshift_in;
   const double mu = 1 - 2.0 * rng.next();
@@ -298,15 +320,15 @@ __device__ __forceinline__ void isotropic_scatter(const StepArgs& A, const GridD
   }
   V[0] = -1 * V[0]; V[1] = -1 * V[1]; V[2] = -1 * V[2];
   const double vdp = (Dn[0] * V[0] + Dn[1] * V[1] + Dn[2] * V[2]);
-  const double vd_out = gamma * (1 - vdp / C_LIGHT);
-  const double f = (1 - gamma * vdp / C_LIGHT / (gamma + 1));
-  p.D[0] = 1.0 / vd_out * (Dn[0] - gamma * V[0] / C_LIGHT * f);
-  p.D[1] = 1.0 / vd_out * (Dn[1] - gamma * V[1] / C_LIGHT * f);
-  p.D[2] = 1.0 / vd_out * (Dn[2] - gamma * V[2] / C_LIGHT * f);
-  const double norm = sqrt(p.D[0] * p.D[0] + p.D[1] * p.D[1] + p.D[2] * p.D[2]);
-  p.D[0] = p.D[0] / norm;
-  p.D[1] = p.D[1] / norm;
-  p.D[2] = p.D[2] / norm;
+  const double vd_out = gamma * (1 - div_c(vdp));
+  const double f = (1 - div_rn(div_c(gamma * vdp), gamma + 1));
+  const double inv_vd = rcp_rn(vd_out);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p.D[k] = inv_vd * (Dn[k] - div_c(gamma * V[k]) * f);
+  const double norm = sqrt_rn(p.D[0] * p.D[0] + p.D[1] * p.D[1] + p.D[2] * p.D[2]);
+  const double inv_norm = rcp_rn(norm);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p.D[k] = div_rn(p.D[k], norm, inv_norm);
   p.e = p.e * vd_out;
   p.nu = p.nu * vd_out;
 }
@@ -508,7 +530,6 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
 // deviates, same path) and adds -w a0 dshift l per segment into the
 // gradient with respect to the (zone, band) absorption factors, where w is
 // the packet's escaping energy times d(loss)/d(its spectrum bin).
-// FAST (mixed form on a homologous grid): the division-free transforms above.
 // discrete diffusion (1D spheres, FP64 expressions), defined with the
 // gamma-ray helpers below
 template <typename OT>
@@ -527,7 +548,7 @@ template <typename OT>
 __device__ int imd_event(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng& rng, double* t_eabs,
                          unsigned long long& n_cap);
 // DD: discrete diffusion on (transport_use_ddmc = 1 IMD or 2 DDMC; 1D, FP64 expressions)
-template <int GRID, typename OT, typename CT, int BATCH, int MODE, bool FAST, int THREADS, int MINB, bool DD = false>
+template <int GRID, typename OT, typename CT, int BATCH, int MODE, int THREADS, int MINB, bool DD = false>
 __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs A, const GridDev G)
 {
   extern __shared__ double s_tal[];  // [5][nz] when A.smem_zones
@@ -550,13 +571,8 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
     t_eabs = base; t_fx = base + nz; t_fy = base + 2 * nz; t_fz = base + 3 * nz; t_fr = base + 4 * nz;
   }
   const OT* __restrict__ opac = reinterpret_cast<const OT*>(A.opac);
-  // the mixed form takes the division-free transforms on homologous grids;
-  // the FP64 form keeps the reference's expressions
-  constexpr bool fast = FAST;
   const int64_t limit = A.max_segments > 0 ? A.max_segments : 10000000;
-  // deviates (per-draw layout) or Philox blocks (word layout) the emission uses
-  uint32_t K = (A.core_radius == 0 ? 2u : 4u) + (A.core_freq > 0 ? 0u : 2u) + 1u;
-  if (FAST) K = (K + 3u) / 4u;
+  uint32_t K = (A.core_radius == 0 ? 2u : 4u) + (A.core_freq > 0 ? 0u : 2u) + 1u;  // deviates the emission draws
   uint32_t step = A.step;
   if constexpr (BATCH) step = *A.step_dev;
   // batch: claimed queue entries [q_next, q_end), the current packet's model,
@@ -658,7 +674,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         pid = (unsigned long long)q_next++;
         m = find_model(A.models, A.n_models, (int64_t)pid);
         const BatchModel& M = A.models[m];
-        K = FAST ? (M.emit_draws + 3u) / 4u : M.emit_draws;
+        K = M.emit_draws;
         rng.init(M.seed, (uint64_t)(M.first_pid + ((int64_t)pid - M.pkt_off)), step, 0);
         BatchZoneOf zf;
         zf.slice = G.r_out;
@@ -666,13 +682,8 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         zf.slice.min = M.r_min;
         zf.slice.right = G.r_out.right + M.zone_off;
         zf.zone_off = M.zone_off;
-        if constexpr (FAST) {
-          DrawWords d{rng};
-          emit_core<GRID>(A, G, p, d, M.core_radius, M.Ep, M.core_cdf, zf);
-        } else {
-          DrawNext d{rng};
-          emit_core<GRID>(A, G, p, d, M.core_radius, M.Ep, M.core_cdf, zf);
-        }
+        DrawNext d{rng};
+        emit_core<GRID>(A, G, p, d, M.core_radius, M.Ep, M.core_cdf, zf);
       } else {
         pid = atomicAdd(A.counters + C_QUEUE, 1ULL);
         if (pid >= (unsigned long long)A.n_packets) break;
@@ -712,13 +723,8 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
           acc_g = 0;
         }
         rng.init(A.seed, (uint64_t)A.first_pid + pid, step, 0);
-        if constexpr (FAST) {
-          DrawWords d{rng};
-          emit_core<GRID>(A, G, p, d, A.core_radius, A.Ep, A.core_cdf, GridZoneOf<GRID>{G});
-        } else {
-          DrawNext d{rng};
-          emit_core<GRID>(A, G, p, d, A.core_radius, A.Ep, A.core_cdf, GridZoneOf<GRID>{G});
-        }
+        DrawNext d{rng};
+        emit_core<GRID>(A, G, p, d, A.core_radius, A.Ep, A.core_cdf, GridZoneOf<GRID>{G});
       }
       // transport::propagate (transport.cpp:202-254): its get_zone of the
       // emitted position is the p.ind emit_core set (x has not moved since)
@@ -765,24 +771,12 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         dd_call = false;
       }
       double d_bn = 0;
-      double rsq, xdotD;
-      if (fast) {
-        rsq = fma(p.x[0], p.x[0], fma(p.x[1], p.x[1], p.x[2] * p.x[2]));
-        xdotD = fma(p.D[0], p.x[0], fma(p.D[1], p.x[1], p.D[2] * p.x[2]));
-      } else {
-        rsq = (p.x[0] * p.x[0] + p.x[1] * p.x[1] + p.x[2] * p.x[2]);
-        xdotD = (p.D[0] * p.x[0] + p.D[1] * p.x[1] + p.D[2] * p.x[2]);
-      }
+      const double rsq = (p.x[0] * p.x[0] + p.x[1] * p.x[1] + p.x[2] * p.x[2]);
+      const double xdotD = (p.D[0] * p.x[0] + p.D[1] * p.x[1] + p.D[2] * p.x[2]);
       int new_ind;
       if constexpr (BATCH) new_ind = get_next_zone_batch(A, G, iz, rsq, xdotD, &d_bn);
-      else new_ind = get_next_zone<GRID, FAST>(G, p.x, p.D, iz, A.core_radius, rsq, xdotD, &d_bn);
-      double dshift;
-      if (fast) {
-        dshift = dshift_fast(A, rsq, xdotD);
-        p.dvds = A.inv_t;
-      } else {
-        dshift = dshift_lab_to_comoving<GRID>(G, p);
-      }
+      else new_ind = get_next_zone<GRID>(G, p.x, p.D, iz, A.core_radius, rsq, xdotD, &d_bn);
+      const double dshift = dshift_lab_to_comoving<GRID>(G, p);
       // a diffusive neighbour (transport.cpp:295-309)
       bool new_cell_ddmc = false;
       double sigma_new = 0, dr_new = 0;
@@ -796,7 +790,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
       }
       // transport::get_opacity (transport_opacity.cpp:268-299)
       const double nu_cmf = p.nu * dshift;
-      const int i_nu = (fast) ? loc_within_fast<true>(A.nu, nu_cmf) : loc_within_fast<false>(A.nu, nu_cmf);
+      const int i_nu = loc_within_fast<false>(A.nu, nu_cmf);
       const OT ab = opac[(size_t)iz * nn + i_nu];
       double a_opac = (double)ab.x;
       const double s_opac = A.omit_scat ? 0.0 : (double)ab.y;
@@ -806,38 +800,14 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         if (A.abs_scale) a_opac *= __ldg(A.abs_scale + (size_t)iz * A.n_bands + band);
       }
       const double op = a_opac + s_opac;
-      double eps = 0;
-      if (!(fast)) eps = (op == 0) ? 0 : a_opac / op;
-      double d_nu;
-      // distance to the bin's edge: only where the segment stops to look up
-      // the next bin, so FP32 in the mixed form
-      if (fast) d_nu = (double)__fdividef((float)(loc_delta(A.nu, i_nu) * A.ct), (float)p.nu);
-      else {
-        d_nu = loc_delta(A.nu, i_nu) / p.nu * C_LIGHT / p.dvds;
-        if (p.dvds == 0) d_nu = INFINITY;
-      }
+      const double eps = absorbed_part(a_opac, op);
+      double d_nu = div_rn(div_rn(loc_delta(A.nu, i_nu), p.nu) * C_LIGHT, p.dvds);
+      if (p.dvds == 0) d_nu = INFINITY;
       if (d_nu < 0) d_nu = -1 * d_nu;
       if (d_nu < d_bn) { d_bn = d_nu; new_ind = p.ind; }
       const double tot_lab = (MODE == 0 ? op : s_opac) * dshift;
-      // mixed form: the segment's Philox block gives tau (53 bits) and the
-      // two interaction tests
-      uint4 blk = make_uint4(0u, 0u, 0u, 0u);
-      double tau_r;
-      if constexpr (FAST) {
-        blk = rng.block();
-        // -log(1 - u) in FP32: log1pf for u < 1/2, logf of the exact FP64
-        // 1 - u above, so the relative error stays ~1e-7 over the whole range
-        const double u = u01(blk.x, blk.y);
-        tau_r = (double)((u < 0.5) ? -log1pf(-(float)u) : -logf((float)(1.0 - u)));
-      } else {
-        tau_r = -1.0 * log(1 - rng.next());
-      }
-      // mixed form: tau is an FP32 deviate, so its distance is formed in FP32
-      // (the hardware's FP32 division, off the FP64 pipe); position and time
-      // stay FP64
-      double d_sc;
-      if constexpr (FAST) d_sc = (double)__fdividef((float)tau_r, (float)tot_lab);
-      else d_sc = tau_r / tot_lab;
+      const double tau_r = -1.0 * log(1 - rng.next());
+      double d_sc = div_rn(tau_r, tot_lab);
       if (tot_lab == 0) d_sc = INFINITY;
       double d_tm = (A.tstop - p.t) * C_LIGHT;
       if (A.steady) d_tm = INFINITY;
@@ -882,8 +852,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
       }
       const double eps_imc = __ldg(A.eps_imc + iz);
       if constexpr (MODE == 0) {
-        if (fast) acc_eabs += this_E * dshift * dshift * a_opac * eps_imc;
-        else acc_eabs += this_E * dshift * (op) * eps * dshift * eps_imc;
+        acc_eabs += this_E * dshift * (op) * eps * dshift * eps_imc;
       }
       if constexpr (MODE == 1) acc_eabs += this_E * dshift * a_opac * dshift * eps_imc;
       if constexpr (MODE != 2) atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
@@ -893,15 +862,12 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         acc_fy += w * p.D[1] * dshift;
         acc_fz += w * p.D[2] * dshift;
         // |x| and x.D before the move: the segment's rsq and xdotD
-        if (fast) acc_fr += w * xdotD * rsqrt(rsq) * dshift;
-        else acc_fr += w * xdotD / sqrt(rsq) * dshift;
+        acc_fr += w * xdotD * rsqrt_nr(rsq) * dshift;
       }
       p.x[0] += this_d * p.D[0];
       p.x[1] += this_d * p.D[1];
       p.x[2] += this_d * p.D[2];
-      constexpr double INV_C = 1.0 / C_LIGHT;
-      if (fast) p.t = p.t + this_d * INV_C;
-      else p.t = p.t + this_d / C_LIGHT;
+      p.t = p.t + div_c(this_d);
       if constexpr (MODE == 1) p.e *= att;
       if (event == 1) {
         if (new_ind == -1) {
@@ -922,16 +888,14 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         ++n_scat;
         int redist = 0;
         if constexpr (MODE == 0) {
-          if (fast) eps = (op == 0) ? 0 : a_opac / op;
-          if (!((FAST ? w01(blk.z) : rng.next()) > eps)) {
-            const double z2 = FAST ? w01(blk.w) : rng.next();
+          if (!(rng.next() > eps)) {
+            const double z2 = rng.next();
             if ((z2 > eps_imc) || A.radiative_eq) redist = 1;
             else fate = ABSORBED;
           }
         }
         if (fate == MOVING) {
-          if (fast) isotropic_scatter_fast<CT>(A, p, rng.block(), redist);
-          else isotropic_scatter<GRID, CT>(A, G, p, rng, redist);
+          isotropic_scatter<GRID, CT>(A, G, p, rng, redist);
         }
       } else {
         fate = STOPPED;
@@ -1106,21 +1070,21 @@ __device__ __forceinline__ void lorentz_transform(const GridDev& G, Pkt& p, int 
   double v[3], dvds;
   get_velocity<GRID>(G, p.ind, p.x, p.D, v, &dvds);
   if (tolab) { v[0] *= -1; v[1] *= -1; v[2] *= -1; }
-  const double beta2 = (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) / C_LIGHT / C_LIGHT;
+  const double beta2 = div_c(div_c(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
   const double vdd = v[0] * p.D[0] + v[1] * p.D[1] + v[2] * p.D[2];
-  const double gamma = 1.0 / sqrt(1 - beta2);
-  const double dshift = gamma * (1 - vdd / C_LIGHT);
+  const double gamma = rcp_sqrt_rn(1 - beta2);
+  const double dshift = gamma * (1 - div_c(vdd));
   p.dvds = dvds;
   p.e *= dshift;
   p.nu *= dshift;
-  const double f = (1 - gamma * vdd / C_LIGHT / (gamma + 1));
-  p.D[0] = 1.0 / dshift * (p.D[0] - gamma * v[0] / C_LIGHT * f);
-  p.D[1] = 1.0 / dshift * (p.D[1] - gamma * v[1] / C_LIGHT * f);
-  p.D[2] = 1.0 / dshift * (p.D[2] - gamma * v[2] / C_LIGHT * f);
+  const double f = (1 - div_rn(div_c(gamma * vdd), gamma + 1));
+  const double inv = rcp_rn(dshift);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p.D[k] = inv * (p.D[k] - div_c(gamma * v[k]) * f);
   const double norm = p.D[0] * p.D[0] + p.D[1] * p.D[1] + p.D[2] * p.D[2];
-  p.D[0] /= norm;
-  p.D[1] /= norm;
-  p.D[2] /= norm;
+  const double y = rcp_rn(norm);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p.D[k] = div_rn(p.D[k], norm, y);
 }
 
 // transport::klein_nishina (transport_opacity.cpp:302-313), x in MeV
@@ -1192,13 +1156,13 @@ __device__ __forceinline__ int ddmc_opacity(const StepArgs& A, const OT* __restr
   const double a_opac = (double)ab.x;
   const double s_opac = A.omit_scat ? 0.0 : (double)ab.y;
   *op = a_opac + s_opac;
-  *eps = (*op == 0) ? 0 : a_opac / *op;
+  *eps = absorbed_part(a_opac, *op);
   return i_nu;
 }
 
 __device__ __forceinline__ double pkt_r(const Pkt& p)
 {
-  return sqrt(p.x[0] * p.x[0] + p.x[1] * p.x[1] + p.x[2] * p.x[2]);
+  return sqrt_rn(p.x[0] * p.x[0] + p.x[1] * p.x[1] + p.x[2] * p.x[2]);
 }
 
 // the zone test of transport::propagate (transport.cpp:219-231)
@@ -1418,20 +1382,24 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
   double r_m = __ldg(G.r_out.right + im);
   if (ii == 0) r_m = G.r_out.min;
   const double r_0 = 0.5 * (r_p + r_m);
-  const double Xi = 1.0 + dx * dx / (12.0 * r_0 * r_0);
-  double geo_factor = r_m * r_m / r_0 / r_0 / Xi;
+  const double y_r0 = rcp_rn(r_0), y_dx = rcp_rn(dx);
+  const double Xi = 1.0 + div_rn(dx * dx, 12.0 * r_0 * r_0);
+  const double y_Xi = rcp_rn(Xi);
+  const double two_thirds_dx = div_rn(2.0 / 3.0, dx, y_dx);
+  double geo_factor = div_rn(div_rn(div_rn(r_m * r_m, r_0, y_r0), r_0, y_r0), Xi, y_Xi);
   const double tau_im1 = sigma_im1 * dxm1;
   const bool ddmc_on_im1 = !(tau_im1 <= A.ddmc_tau);
+  const double far_side = rcp_any(sigma_i * dx + 2.0 * lambda_ddmc);
   double sigma_leak_left;
-  if (ddmc_on_im1) sigma_leak_left = (2.0 / 3.0 / dx) * (1.0 / (sigma_i * dx + sigma_im1 * dxm1)) * geo_factor;
-  else sigma_leak_left = (2.0 / 3.0 / dx) * (1.0 / (sigma_i * dx + 2.0 * lambda_ddmc)) * geo_factor;
-  geo_factor = r_p * r_p / r_0 / r_0 / Xi;
+  if (ddmc_on_im1) sigma_leak_left = two_thirds_dx * rcp_any(sigma_i * dx + sigma_im1 * dxm1) * geo_factor;
+  else sigma_leak_left = two_thirds_dx * far_side * geo_factor;
+  geo_factor = div_rn(div_rn(div_rn(r_p * r_p, r_0, y_r0), r_0, y_r0), Xi, y_Xi);
   const double tau_ip1 = sigma_ip1 * dxp1;
   const bool ddmc_on_ip1 = !(tau_ip1 <= A.ddmc_tau);
   double sigma_leak_right;
-  if (ddmc_on_ip1) sigma_leak_right = (2.0 / 3.0 / dx) * (1.0 / (sigma_i * dx + sigma_ip1 * dxp1)) * geo_factor;
-  else sigma_leak_right = (2.0 / 3.0 / dx) * (1.0 / (sigma_i * dx + 2.0 * lambda_ddmc)) * geo_factor;
-  if (ip == ii) sigma_leak_right = (2.0 / 3.0 / dx) * (1.0 / (sigma_i * dx + 2.0 * lambda_ddmc)) * geo_factor;
+  if (ddmc_on_ip1) sigma_leak_right = two_thirds_dx * rcp_any(sigma_i * dx + sigma_ip1 * dxp1) * geo_factor;
+  else sigma_leak_right = two_thirds_dx * far_side * geo_factor;
+  if (ip == ii) sigma_leak_right = two_thirds_dx * far_side * geo_factor;
   if (ii == 0) sigma_leak_left = 0.0;
   const double sigma_leak_tot = sigma_leak_left + sigma_leak_right;
   const double xi = rng.next();
@@ -1460,7 +1428,7 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
   if ((d_sc < d_leak) && (d_sc < d_stay)) { event = 0; this_d = d_sc; }
   else if (d_leak < d_stay) { event = 1; this_d = d_leak; }
   else { event = 2; this_d = d_stay; }
-  const double this_dt = this_d / C_LIGHT;
+  const double this_dt = div_c(this_d);
   p.t += this_dt;
   dt_remaining -= this_dt;
   atomicAdd(A.J + (size_t)p.ind * nj, p.e * this_d);
@@ -1487,7 +1455,7 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
     dt_remaining = -1.0;
     fate = STOPPED;
   } else {
-    const double P_leak_left = sigma_leak_left / sigma_leak_tot;
+    const double P_leak_left = div_rn(sigma_leak_left, sigma_leak_tot);
     const double xi2 = rng.next();
     if (xi2 <= P_leak_left) {
       p.ind--;
@@ -1495,9 +1463,10 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
       double dr = rr - r_m;
       if (ddmc_on_im1) dr += rng.next() * dxm1;
       else dr *= (1.0 + push);
-      p.x[0] -= p.x[0] / rr * dr;
-      p.x[1] -= p.x[1] / rr * dr;
-      p.x[2] -= p.x[2] / rr * dr;
+      const double y = rcp_rn(rr);
+      p.x[0] -= div_rn(p.x[0], rr, y) * dr;
+      p.x[1] -= div_rn(p.x[1], rr, y) * dr;
+      p.x[2] -= div_rn(p.x[2], rr, y) * dr;
       if (!ddmc_on_im1) {
         leaked2imc = true;
         lorentz_transform<0>(G, p, 0);
@@ -1512,9 +1481,10 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
       double dr = r_p - rr;
       if (ddmc_on_ip1) dr += rng.next() * dxp1;
       else dr *= (1.0 + push);
-      p.x[0] += p.x[0] / rr * dr;
-      p.x[1] += p.x[1] / rr * dr;
-      p.x[2] += p.x[2] / rr * dr;
+      const double y = rcp_rn(rr);
+      p.x[0] += div_rn(p.x[0], rr, y) * dr;
+      p.x[1] += div_rn(p.x[1], rr, y) * dr;
+      p.x[2] += div_rn(p.x[2], rr, y) * dr;
       if (!ddmc_on_ip1) {
         leaked2imc = true;
         lorentz_transform<0>(G, p, 0);
@@ -1528,8 +1498,8 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
   // advection and the adiabatic loss (discrete_diffusion.cpp:371-397)
   double zone_vel[3], dvds;
   get_velocity<0>(G, p.ind, p.x, p.D, zone_vel, &dvds);
-  const double vel = sqrt(zone_vel[0] * zone_vel[0] + zone_vel[1] * zone_vel[1] + zone_vel[2] * zone_vel[2]);
-  const double v_over_r = vel / pkt_r(p);
+  const double vel = sqrt_rn(zone_vel[0] * zone_vel[0] + zone_vel[1] * zone_vel[1] + zone_vel[2] * zone_vel[2]);
+  const double v_over_r = div_rn(vel, pkt_r(p));
   const double dlnrhodt = dvds + 2.0 * v_over_r;
   const double doppler_shift_ddmc = (1.0 - dlnrhodt * this_dt / 3.0);
   lorentz_transform<0>(G, p, 0);
@@ -1983,13 +1953,12 @@ int launch_fp64_t(const StepArgs& a0, const GridDev& g, int blocks_per_sm, int n
   return 1;
 }
 
-template <int GRID, typename OT, typename CT, int BATCH, int THREADS, int MINB, int MODE = 0,
-          bool FAST = (sizeof(OT) == sizeof(float2)), bool DD = false>
+template <int GRID, typename OT, typename CT, int BATCH, int THREADS, int MINB, int MODE = 0, bool DD = false>
 int launch_kernel_t(const StepArgs& a, const GridDev& g, int blocks_per_sm, int num_sms, int64_t total,
                     cudaStream_t s)
 {
   const size_t smem = a.smem_zones ? (size_t)5 * g.nzones * sizeof(double) : 0;
-  auto kern = propagate_kernel<GRID, OT, CT, BATCH, MODE, FAST, THREADS, MINB, DD>;
+  auto kern = propagate_kernel<GRID, OT, CT, BATCH, MODE, THREADS, MINB, DD>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem);
@@ -2003,11 +1972,6 @@ int launch_kernel_t(const StepArgs& a, const GridDev& g, int blocks_per_sm, int 
   return 1;
 }
 
-// Single-context shapes: the FP64 form runs best with 256 x 4 (64
-// registers; Type Ia step 1753 ms vs 1788 ms at 128 x 8); the mixed form on
-// 1D grids is propagate_mixed_kernel (SED_MIXED_THREADS x SED_MIXED_MINB);
-// on 3D grids the mixed form runs 128 x 7 (64^3 cells, 2e7 packets: packet
-// kernel 572 ms vs 583 ms at 256 x 3).
 // the FP64 kernel's grids: homologous, at a time its reciprocals cover
 bool fp64_ok(const StepArgs& a, const GridDev& g)
 {
@@ -2042,12 +2006,12 @@ int launch_propagate_t(const StepArgs& a, const GridDev& g, int num_sms, cudaStr
   // discrete diffusion (1D): the reference's expressions in both forms
   if constexpr (GRID == 0) {
     if (a.use_ddmc == 1 || a.use_ddmc == 2)
-      return launch_kernel_t<0, OT, CT, 0, 256, 4, 0, false, true>(a, g, 0, num_sms, a.n_packets, s);
+      return launch_kernel_t<0, OT, CT, 0, 256, 4, 0, true>(a, g, 0, num_sms, a.n_packets, s);
   }
   // mixed tables on a grid with a tabulated velocity field: the reference's
   // expressions (the division-free transforms assume v = x / t)
   if (sizeof(OT) == sizeof(float2) && !g.homologous)
-    return launch_kernel_t<GRID, OT, CT, 0, 256, 4, 0, false>(a, g, 0, num_sms, a.n_packets, s);
+    return launch_kernel_t<GRID, OT, CT, 0, 256, 4>(a, g, 0, num_sms, a.n_packets, s);
   if constexpr (sizeof(OT) == sizeof(float2)) {
     if constexpr (GRID == 0) return launch_mixed_t<0, SED_MIXED_THREADS, SED_MIXED_MINB>(a, g, 0, num_sms, a.n_packets, s);
     else return launch_cart(a, g, num_sms, s);
@@ -2098,6 +2062,15 @@ bool mixed_1d_path(const StepArgs& a, const GridDev& g)
 }
 
 bool fp64_path(const StepArgs& a, const GridDev& g) { return fp64_ok(a, g); }
+
+void set_grid_time(GridDev& g, double t_grid)
+{
+  g.t_grid = t_grid;
+  g.inv_t = g.inv_t_lo = 0;
+  if (!(t_grid > 1e-100 && t_grid < 1e100)) return;
+  g.inv_t = 1.0 / t_grid;
+  g.inv_t_lo = std::fma(-t_grid, g.inv_t, 1.0) * g.inv_t;
+}
 
 void set_grid_time(StepArgs& a, double t_grid)
 {
