@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_cart_kernel(const Ste
   const int nn = A.nu.n, nyz = G.ny * G.nz;
   const int64_t rep_off = (A.n_rep > 0) ? (int64_t)(blockIdx.x % A.n_rep) * 5 * G.nzones : -1;
   const int nj = A.store_Jnu ? nn : 1;
+  double* __restrict__ J = tally_J(A, G.nzones, nj);
   const float2* __restrict__ opac = reinterpret_cast<const float2*>(A.opac);
   const int32_t limit = A.max_segments > 0 ? A.max_segments : 10000000;
   const uint32_t K = ((A.core_radius == 0 ? 2u : 4u) + (A.core_freq > 0 ? 0u : 2u) + 1u + 3u) / 4u;
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_cart_kernel(const Ste
     else { event = 2; this_d = d_tm; }
     // tallies (transport.cpp:361-392)
     const double this_E = p.e * this_d;
-    atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
+    atomicAdd(J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
     const double eps_imc = __ldg(A.eps_imc + iz);
     const double ed = this_E * dshift;
     s_acc[0][tid] += ed * dshift * a_opac * eps_imc;

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_fp64_kernel(const Ste
   const int nz = G.nzones;
   const int nn = A.nu.n;
   const int nj = A.store_Jnu ? nn : 1;
+  double* __restrict__ J = tally_J(A, G.nzones, nj);
   if (A.smem_zones)
     for (int i = tid; i < 5 * nz; i += THREADS) s_tal[i] = 0.0;
 #pragma unroll
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_fp64_kernel(const Ste
     const double this_E = p.e * this_d;
     const double eps_imc = __ldg(A.eps_imc + iz);
     const double ed = this_E * dshift;
-    atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
+    atomicAdd(J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
     s_acc[0][tid] += ed * a_opac * dshift * eps_imc;
     if (A.tally_forces) {
       const double w = ed * op * dshift;

@@ -432,6 +432,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
   const int nz = G.nzones;
   const int nn = A.nu.n;
   const int nj = A.store_Jnu ? nn : 1;
+  double* __restrict__ J = tally_J(A, G.nzones, nj);
   if (A.smem_zones)
     for (int i = threadIdx.x; i < 5 * nz; i += blockDim.x) s_tal[i] = 0.0;
   __syncthreads();
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_mixed_kernel(const St
     const double ed = this_E * dshift;
     double* sa = &s_acc[SLOTS == 2 ? (acc & 1) : 0][0][tid];
     sa[0] = fma(ed * dshift * (double)a_f, eps_imc, sa[0]);
-    atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
+    atomicAdd(J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
     if (A.tally_forces) {
       const double wd = ed * (double)op_f * dshift;
       sa[THREADS] = fma(wd, p.D[0], sa[THREADS]);

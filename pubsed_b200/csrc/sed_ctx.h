@@ -121,7 +121,8 @@ struct sed_ctx {
   // tables
   bool have_opacity = false;
   DevBuf<unsigned char> d_opac, d_cdf, d_cdf_coarse;
-  DevBuf<double> d_zone_rep;          // [n_rep][5][nz] zone-scalar tally copies of the 1D mixed kernel
+  DevBuf<double> d_zone_rep;          // [n_rep][5][nz] zone-scalar tally copies of the 1D kernels
+  DevBuf<double> d_J_rep;             // [n_rep_J][nz*nj] copies of a small mean-intensity tally
   DevBuf<double> d_rho_scale;         // per-zone extinction factors of the last scaling
   DevBuf<unsigned char> d_opac_base;  // the built {abs, scat} tables while scaled ones are in d_opac
   bool opac_base_valid = false;       // d_opac_base holds the tables of the last build or load
@@ -262,6 +263,8 @@ int enqueue_opacity(sed_ctx* c, double dt);
 cudaError_t pack_bins(sed_ctx* c);
 // the zone-scalar tallies of a step in copies (zeroed), for the packet and finish kernels
 int zone_tally_copies(sed_ctx* c, StepArgs& A);
+// the same for the mean intensity, where it is small
+int J_tally_copies(sed_ctx* c, StepArgs& A);
 StepArgs make_step_args(sed_ctx* c, double dt, int64_t n_emit);
 GridDev make_grid_dev(sed_ctx* c);
 

@@ -44,6 +44,8 @@ struct StepArgs {
   const double* imd_p;        // IMD: [4][nz] hop up, hop down, stay, absorb probabilities of the step
   int32_t smem_zones;         // 1: per-block shared-memory zone tallies
   int32_t n_rep;              // >0 (and smem_zones 0): zone-scalar tallies in n_rep global copies
+  int32_t n_rep_J;            // >0: the mean intensity tallied in n_rep_J global copies
+  double* J_rep;              // [n_rep_J][J's size], summed into J by the finish kernel
   double* zone_rep;           // [n_rep][5][nz] e_abs, fx, fy, fz, fr copies, summed by the finish kernel
   DevLoc nu, st, sn, sm, sp;  // frequency grid and spectrum grids
   int64_t a1, a2, a3;         // spectrum strides

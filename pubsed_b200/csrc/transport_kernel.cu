@@ -207,6 +207,12 @@ __device__ __forceinline__ void comoving_to_lab(const GridDev& G, Pkt& p)
   for (int k = 0; k < 3; ++k) p.D[k] = div_rn(p.D[k], norm, y);
 }
 
+// the block's mean-intensity tally: one of the copies where there are any
+__device__ __forceinline__ double* tally_J(const StepArgs& A, int nz, int nj)
+{
+  return (A.n_rep_J > 0) ? A.J_rep + (size_t)(blockIdx.x % A.n_rep_J) * nz * nj : A.J;
+}
+
 // ----------------------------------------------------------- batches
 // get_next_zone of grid_1D_sphere for a zone of one model of a batch.  The
 // model's walls sit in the concatenated r_out array; per zone the host has
@@ -536,7 +542,7 @@ template <typename OT>
 __device__ bool ddmc_zone(const StepArgs& A, const GridDev& G, const OT* __restrict__ opac, Pkt& p);
 template <typename OT, typename CT>
 __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restrict__ opac, Pkt& p, PacketRng& rng,
-                          double& dt_remaining, double& acc_eabs, unsigned long long& n_scat,
+                          double& dt_remaining, double* J, double& acc_eabs, unsigned long long& n_scat,
                           unsigned long long& n_cap);
 __device__ void ddmc_move_across(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng& rng, int new_ind,
                                  double sigma_i, double dr);
@@ -545,7 +551,7 @@ __device__ __forceinline__ int ddmc_opacity(const StepArgs& A, const OT* __restr
                                             double* op, double* eps);
 
 template <typename OT>
-__device__ int imd_event(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng& rng, double* t_eabs,
+__device__ int imd_event(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng& rng, double* t_eabs, double* J,
                          unsigned long long& n_cap);
 // DD: discrete diffusion on (transport_use_ddmc = 1 IMD or 2 DDMC; 1D, FP64 expressions)
 template <int GRID, typename OT, typename CT, int BATCH, int MODE, int THREADS, int MINB, bool DD = false>
@@ -555,6 +561,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
   const int nz = G.nzones;
   const int nn = A.nu.n;
   const int nj = A.store_Jnu ? nn : 1;
+  double* __restrict__ J = tally_J(A, nz, nj);
   if (A.smem_zones) {
     for (int i = threadIdx.x; i < 5 * nz; i += blockDim.x) s_tal[i] = 0.0;
     __syncthreads();
@@ -761,11 +768,11 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         // in a diffusive zone takes a diffusion event instead of a segment
         if (ddmc_zone<OT>(A, G, opac, p)) {
           if (A.use_ddmc == 1) {  // one IMD call (transport.cpp:236-237)
-            fate = imd_event<OT>(A, G, p, rng, t_eabs, n_imdcap);
+            fate = imd_event<OT>(A, G, p, rng, t_eabs, J, n_imdcap);
             continue;
           }
           if (!dd_call) { dd_rem = A.tstop - p.t; dd_call = true; }
-          fate = ddmc_event<OT, CT>(A, G, opac, p, rng, dd_rem, acc_eabs, n_scat, n_ddcap);
+          fate = ddmc_event<OT, CT>(A, G, opac, p, rng, dd_rem, J, acc_eabs, n_scat, n_ddcap);
           continue;
         }
         dd_call = false;
@@ -855,7 +862,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
         acc_eabs += this_E * dshift * (op) * eps * dshift * eps_imc;
       }
       if constexpr (MODE == 1) acc_eabs += this_E * dshift * a_opac * dshift * eps_imc;
-      if constexpr (MODE != 2) atomicAdd(A.J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
+      if constexpr (MODE != 2) atomicAdd(J + (size_t)iz * nj + (A.store_Jnu ? i_nu : 0), this_E);
       if (MODE != 2 && A.tally_forces) {
         const double w = this_E * dshift * op;
         acc_fx += w * p.D[0] * dshift;
@@ -1010,6 +1017,17 @@ __global__ void finish_zones_kernel(const StepArgs A, const double* __restrict__
       for (int r = 0; r < A.n_rep; ++r) sum += A.zone_rep[((size_t)r * 5 + threadIdx.x) * nz + iz];
       double* dst[5] = {A.e_abs, A.fx, A.fy, A.fz, A.fr};
       dst[threadIdx.x][iz] += sum;
+    }
+    __syncthreads();
+  }
+  if (A.n_rep_J > 0) {
+    const int nj = A.store_Jnu ? A.nu.n : 1;
+    const size_t stride = (size_t)nz * nj;
+    for (int j = threadIdx.x; j < nj; j += blockDim.x) {
+      const size_t k = (size_t)iz * nj + j;
+      double sum = 0;
+      for (int r = 0; r < A.n_rep_J; ++r) sum += A.J_rep[r * stride + k];
+      A.J[k] += sum;
     }
     __syncthreads();
   }
@@ -1256,7 +1274,7 @@ __device__ void ddmc_move_across(const StepArgs& A, const GridDev& G, Pkt& p, Pa
 // reference; the hop loop, unbounded there, gives up after 2^24 hops
 // (counted, SED_ERR_LIMIT).
 template <typename OT>
-__device__ int imd_event(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng& rng, double* t_eabs,
+__device__ int imd_event(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng& rng, double* t_eabs, double* J,
                          unsigned long long& n_cap)
 {
   const int nz = G.nzones, nn = A.nu.n;
@@ -1275,7 +1293,7 @@ __device__ int imd_event(const StepArgs& A, const GridDev& G, Pkt& p, PacketRng&
     if (p.ind == -2) return ESCAPED;
     const int i = p.ind;
     atomicAdd(t_eabs + i, p.e * __ldg(P_ab + i));
-    atomicAdd(A.J + (size_t)i * nj, p.e * __ldg(P_st + i) * dt * C_LIGHT);
+    atomicAdd(J + (size_t)i * nj, p.e * __ldg(P_st + i) * dt * C_LIGHT);
     const double P_diff = __ldg(P_up + i) + __ldg(P_dn + i);
     const double P_stay = __ldg(P_ab + i) + __ldg(P_st + i);
     const double r1 = rng.next();
@@ -1361,7 +1379,7 @@ __global__ void imd_probabilities_kernel(const GridDev G, const double* __restri
 // 65536 re-emissions that stay in the same bin (counted).
 template <typename OT, typename CT>
 __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restrict__ opac, Pkt& p, PacketRng& rng,
-                          double& dt_remaining, double& acc_eabs, unsigned long long& n_scat,
+                          double& dt_remaining, double* J, double& acc_eabs, unsigned long long& n_scat,
                           unsigned long long& n_cap)
 {
   const int nz = G.nzones, nn = A.nu.n;
@@ -1431,7 +1449,7 @@ __device__ int ddmc_event(const StepArgs& A, const GridDev& G, const OT* __restr
   const double this_dt = div_c(this_d);
   p.t += this_dt;
   dt_remaining -= this_dt;
-  atomicAdd(A.J + (size_t)p.ind * nj, p.e * this_d);
+  atomicAdd(J + (size_t)p.ind * nj, p.e * this_d);
   acc_eabs += (p.e * dshift) * this_d * sigma_i * eps_i;
   if (event == 0) {
     ++n_scat;
