@@ -832,6 +832,11 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
     launches += launch_imd_probabilities(G, c->d_planck.p, dt, c->d_imd_p.p, c->stream);
     A.imd_p = c->d_imd_p.p;
   }
+  if (c->tp.use_ddmc == 2) {
+    CK(c->d_dd_geo.resize(3 * nz));
+    launches += launch_ddmc_geometry(G, c->d_dd_geo.p, c->stream);
+    A.dd_geo = c->d_dd_geo.p;
+  }
   if (mixed_1d_path(A, G) && n_emit > 0) {  // core packets emitted ahead of the packet kernel
     CK(c->d_em_state.resize((size_t)n_emit * 9));
     CK(c->d_em_ind.resize((size_t)n_emit));
@@ -1200,7 +1205,7 @@ void sed_ctx_destroy(sed_ctx* c)
   c->d_q_ind.release(); c->d_reject.release(); c->d_q_n.release();
   c->d_rec_type.release(); c->d_census_state.release(); c->d_census_ind.release(); c->d_census_type.release();
   c->d_q_type.release(); c->d_cmp.release(); c->d_scan_tmp.release(); c->d_cmp_count.release();
-  c->d_rho_scale.release(); c->d_opac_base.release(); c->d_imd_p.release(); c->d_zone_rep.release(); c->d_J_rep.release();
+  c->d_rho_scale.release(); c->d_opac_base.release(); c->d_imd_p.release(); c->d_dd_geo.release(); c->d_zone_rep.release(); c->d_J_rep.release();
   c->d_em_state.release(); c->d_em_ind.release(); c->d_em_tau.release();
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

@@ -156,6 +156,7 @@ struct sed_ctx {
   int guide_n = 0;
   int chunk_zones = 0;  // zones per opacity-build pass (bounds the FP64/LTE scratch)
   int opacity_launches = 0;
+  DevBuf<double> d_dd_geo; // DDMC zone factors of the step [3][nz]
   DevBuf<double> d_imd_p;  // IMD probabilities of the step [4][nz]
   // core packets emitted ahead of the mixed-form 1D kernel: state [9][n], zone, first optical depth
   DevBuf<double> d_em_state;

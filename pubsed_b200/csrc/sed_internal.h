@@ -41,6 +41,7 @@ struct StepArgs {
   int32_t max_segments;
   int32_t use_ddmc;           // 1: IMD, 2: DDMC in diffusive zones (1D)
   double ddmc_tau;            // transport_ddmc_tau_threshold
+  const double* dd_geo;       // DDMC: [3][nz] 2/3/dx and the wall factors of the leakage opacities
   const double* imd_p;        // IMD: [4][nz] hop up, hop down, stay, absorb probabilities of the step
   int32_t smem_zones;         // 1: per-block shared-memory zone tallies
   int32_t n_rep;              // >0 (and smem_zones 0): zone-scalar tallies in n_rep global copies
@@ -216,6 +217,7 @@ bool cart_path(const StepArgs& a, const GridDev& g);
 int launch_pushed_walls(const DevLoc& ax, double2* out, cudaStream_t s);
 // IMD probabilities of the step (transport::compute_diffusion_probabilities)
 // from the zone Planck means into out[4][nz]
+int launch_ddmc_geometry(const GridDev& g, double* out, cudaStream_t s);
 int launch_imd_probabilities(const GridDev& g, const double* planck, double dt, double* out, cudaStream_t s);
 // zone-scalar tally normalisation (reduce_radiation) and steady-state rescale
 int launch_finish(const StepArgs& a, const GridDev& g, const double* vol, int64_t nspec, cudaStream_t s);
