@@ -543,7 +543,7 @@ def main_adjoint(args, rank: int, world: int, local: int):
            "e2e": {"value": n / e2e, "unit": UNIT, "h2d_bytes_per_step": int(theta.nbytes + g.nbytes),
                    "d2h_bytes_per_step": int(flux.nbytes + click.nbytes + grad.nbytes), "ms_per_step": e2e * 1e3},
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                        "traffic": None, "kernel": "propagate_kernel (weighted forward)", "kernel_ms": ms_k,
+                        "traffic": None, "kernel": "propagate_diff_kernel (weighted forward)", "kernel_ms": ms_k,
                         "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},
            "clocks": clk.summary()}
     if not args.no_cpu_baseline:
@@ -833,7 +833,7 @@ def main():
                 "ms_per_step": e2e_t * 1e3},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic,
-                     "kernel": "propagate_mixed_kernel" if w.zones.type != abi.GRID_3D_CART else "propagate_kernel",
+                     "kernel": "propagate_mixed_kernel" if w.zones.type != abi.GRID_3D_CART else "propagate_cart_kernel",
                      "kernel_ms": kern_ms,
                      "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},
         "clocks": clk.summary(),
