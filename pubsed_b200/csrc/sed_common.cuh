@@ -216,7 +216,8 @@ struct DevLoc {
   const double* right;  // device pointer, n walls
   float inv_step;       // log grids: 1/log2(1+del); lin grids: 1/del (index estimate only)
   float lmin_step;      // log grids: log2(min) * inv_step (index estimate without a division)
-  float inv_min;        // log grids: 1/min (the mixed form's estimate, without cancellation)
+  float inv_min;        // log grids: 1/min (loc_within_mixed's estimate, without cancellation)
+  float margin;         // how far from a wall that estimate decides alone, in bins (lookup_margin)
 };
 
 __device__ __forceinline__ int upper_bound_dev(const double* __restrict__ a, int n, double v)
@@ -333,15 +334,14 @@ __device__ __forceinline__ int loc_within_fast(const DevLoc& g, double x)
   return i;
 }
 
-// The mixed form's bin lookup on log and linear grids: the FP32 index
+// The packet kernels' bin lookup on log and linear grids: the FP32 index
 // estimate (log2(x/min)/log2(1+del), or (x-min)/del) is the bin unless it
-// lies within a margin of a wall, where the walls decide (loc_within_fast).
-// The estimate's error is below ~4e-7 n bins for an n-bin grid (__log2f's
-// 2 ulp, the FP32 roundings of x/min, 1/log2(1+del) and an index below n):
-// 1.5e-3 of a bin on the 4096-bin Type Ia grid, against a margin of
-// max(1/64, n 2^-18) of a bin, ten times larger.  The answer is the bin the
+// lies within the grid's margin of a wall, where the walls decide
+// (loc_within_fast).  The margin is at least twice what the estimate can be
+// off by (lookup_margin, formed with the grid), so the answer is the bin the
 // walls give, and the wall loads, two dependent memory round trips, are
-// left out for ~97% of the Type Ia lookups.
+// left out for ~97% of the Type Ia lookups (4096 bins over a factor of 100:
+// off by at most 3e-3 of a bin, margin 1/64).
 __device__ __forceinline__ int loc_within_mixed(const DevLoc& g, double x)
 {
   if (g.n == 1) return 0;
@@ -350,8 +350,7 @@ __device__ __forceinline__ int loc_within_mixed(const DevLoc& g, double x)
   est = fminf(fmaxf(est, 0.0f), (float)g.n - 0.5f);  // below the grid: bin 0; above: bin n-1
   const int i = (int)est;
   const float fr = est - (float)i;
-  const float margin = fmaxf(0.015625f, (float)g.n * 3.814697265625e-6f);
-  if (fr > margin && fr < 1.0f - margin) return i;
+  if (fr > g.margin && fr < 1.0f - g.margin) return i;
   return loc_within_fast<true>(g, x);
 }
 

@@ -62,6 +62,7 @@ struct DevBuf {
 struct HostLoc {
   int type = 0;
   double min = 0, del = 0;
+  float margin = 1;  // lookup_margin
   std::vector<double> x;
   int n() const { return (int)x.size(); }
   double left(int i) const { return i == 0 ? min : x[i - 1]; }
@@ -85,6 +86,37 @@ struct HostLoc {
   int within(double v) const { const int i = locate(v); return i == n() ? n() - 1 : i; }
 };
 
+// The distance from a wall, in bins, beyond which loc_within_mixed's FP32
+// index estimate is the bin: 1/64, or more where twice the estimate's error is
+// more; 0.5 and above leaves every lookup to the walls.  On a log grid the
+// estimate log2f(float(x) inv_min) inv_step is off by the three roundings of
+// its argument (3 2^-24 / ln 2 in the logarithm), __log2f's error (2^-22 below
+// a logarithm of 1, two ulp above) and the roundings of inv_step and of the
+// index: 2^-22 (1.1 + max(1, R)) inv_step + 2^-23 n for n bins over a range
+// of R = log2(max/min).  Narrow grids of many bins have a large inv_step: 4096
+// bins over 2 % take 0.14.  A linear grid's estimate is off by a few 2^-24 n,
+// and by what x - min loses.  To either comes how far the walls themselves lie
+// from where min and del put them.
+inline float lookup_margin(const HostLoc& h)
+{
+  const int n = h.n();
+  if (n < 2 || !(h.del > 0) || (h.type != LOC_LOG && h.type != LOC_LIN)) return 1.f;
+  const double top = h.x[n - 1];
+  double off = 0, err = n * 0x1p-23;
+  if (h.type == LOC_LOG) {
+    if (!(h.min > 1e-37 && top < 1e37)) return 1.f;  // 1/min and x as floats
+    const double inv_step = 1.0 / std::log2(1.0 + h.del);
+    for (int i = 0; i + 1 < n; ++i)
+      off = std::max(off, std::fabs(std::log2(h.x[i] / h.min) * inv_step - (i + 1)));
+    err += 0x1p-22 * (1.1 + std::max(1.0, std::log2(top / h.min))) * inv_step;
+  } else {
+    for (int i = 0; i + 1 < n; ++i) off = std::max(off, std::fabs((h.x[i] - h.min) / h.del - (i + 1)));
+    err += 0x1p-52 * (std::fabs(h.min) + std::fabs(top)) / h.del;
+  }
+  const double m = std::max({1.0 / 64, n * 0x1p-18, 2 * err}) + off;
+  return m < 1 ? (float)m : 1.f;  // also when a wall is no number
+}
+
 inline HostLoc host_loc(const sed_locate_grid& g)
 {
   HostLoc h;
@@ -92,6 +124,7 @@ inline HostLoc host_loc(const sed_locate_grid& g)
   h.min = g.min;
   h.del = g.del;
   h.x.assign(g.right, g.right + g.n);
+  h.margin = lookup_margin(h);
   return h;
 }
 
@@ -269,6 +302,7 @@ inline DevLoc dev_loc(const HostLoc& h, const DevBuf<double>& d)
   else if (h.type == LOC_LIN && h.del > 0) g.inv_step = (float)(1.0 / h.del);
   g.lmin_step = (h.type == LOC_LOG && h.min > 0) ? (float)(std::log2(h.min) * g.inv_step) : 0.f;
   g.inv_min = (h.type == LOC_LOG && h.min > 0) ? (float)(1.0 / h.min) : 0.f;
+  g.margin = h.margin;
   return g;
 }
 
