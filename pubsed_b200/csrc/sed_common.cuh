@@ -147,20 +147,34 @@ __device__ __forceinline__ double rcp_nr(double a)
 
 // ------------------------------------------- IEEE results without branches
 // Division, reciprocal and square root rounded as IEEE 754 rounds them, for
-// operands and results in the normal range (and a zero dividend or radicand),
-// as straight-line code: CUDA's own branch to a special-case path, and the
-// compiler overlaps nothing across those branches.  The methods are
-// Markstein's (IA-64 and Elementary Functions, 2000, chapters 8 and 9): a
+// operands and results in the normal range, dividends and radicands from 2^-969
+// (the residuals' last bit is 2^-105 of them; below it hard cases may be an ulp
+// off) and a zero dividend or radicand, as straight-line code: CUDA's own
+// branch to a special-case path, and the compiler overlaps nothing across those
+// branches.  The methods are Markstein's (IA-64 and Elementary Functions, 2000, chapters 8 and 9): a
 // reciprocal within an ulp of 1/b becomes the rounded one by one more Newton
 // step with an exact residual, a quotient (root) within an ulp becomes the
-// rounded one by one correction with an exact residual.  Both theorems except
-// a divisor whose 53 bits are all ones.
+// rounded one by one correction with an exact residual.  The step to the
+// reciprocal has one exception, a divisor whose 53 bits are all ones: 1/b lies
+// 2^-53 of half a unit above the midpoint of a power of two and its successor,
+// and from the power of two the step ends in a tie.  1 - 2^-53 is such a
+// divisor, and a Doppler factor, the length of a direction or 1 - beta^2 can
+// take it, so its reciprocal is completed below.  (A root has the like at
+// 4^k (1 - 2^-53), where the step is right from the power of two, which the
+// hardware's approximation gives; every exponent of it from 2^-968 is tested.)
+
+// z = 1/b rounded, but for a b of all ones z may be the power of two below
+__device__ __forceinline__ double rcp_of_ones(double z, double b)
+{
+  const int m = __double2loint(b) & (__double2hiint(b) | (int)0xFFF00000);
+  return __hiloint2double(__double2hiint(z), __double2loint(z) | (int)(m == -1));
+}
 
 // 1/b
 __device__ __forceinline__ double rcp_rn(double b)
 {
   const double y = rcp_nr(b);
-  return fma(fma(-b, y, 1.0), y, y);
+  return rcp_of_ones(fma(fma(-b, y, 1.0), y, y), b);
 }
 
 // a/b from y = rcp_rn(b)
@@ -193,7 +207,7 @@ __device__ __forceinline__ double rcp_sqrt_rn(double a)
 {
   double y;
   const double s = sqrt_rn(a, &y);
-  return fma(fma(-s, y, 1.0), y, y);
+  return rcp_of_ones(fma(fma(-s, y, 1.0), y, y), s);
 }
 
 // a/b for a divisor known ahead, zh + zl its reciprocal to twice the precision
