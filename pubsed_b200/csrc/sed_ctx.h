@@ -20,15 +20,18 @@ struct DevBuf {
   T* p = nullptr;
   size_t n = 0;    // elements in use
   size_t cap = 0;  // elements allocated
-  // A buffer under 1 GiB stays when the new size fills 7/8 of it, and one that
+  // A buffer under 1 GiB stays when the new size fills 3/4 of it, and one that
   // grows takes 1/8 more than asked for where there is room: packet counts
   // change from step to step (escapes, decay packets), and freeing and
   // allocating the lists of 1e6 carried packets took 8.5 of a step's 16 ms.
+  // The two lines are far enough apart that counts which swing by up to 15 %
+  // stay in the buffer that the first growth made (with 7/8 a fall of 1.6 %
+  // after a growth left it again).
   cudaError_t resize(size_t m)
   {
     if (m == n && p) return cudaSuccess;
     const bool small = m <= (size_t(1) << 30) / sizeof(T);
-    if (p && m > 0 && small && m <= cap && m >= cap - cap / 8) {
+    if (p && m > 0 && small && m <= cap && m >= cap - cap / 4) {
       n = m;
       return cudaSuccess;
     }
