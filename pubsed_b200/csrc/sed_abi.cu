@@ -981,7 +981,7 @@ int sed_solve_temperature(sed_ctx* c, int32_t set_Tgas_to_Trad, double* T_gas, i
   CK(c->d_temp_bad.resize(1));
   A.n_unsolved = c->d_temp_bad.p;
   CK(cudaMemsetAsync(c->d_temp_bad.p, 0, sizeof(int32_t), c->stream));
-  launch_temperature(A, c->stream);
+  launch_temperature(A, c->num_sms, c->stream);
   CK(cudaGetLastError());
   int32_t bad = 0;
   CK(cudaMemcpyAsync(&bad, c->d_temp_bad.p, sizeof bad, cudaMemcpyDeviceToHost, c->stream));

@@ -253,8 +253,8 @@ struct TemperatureArgs {
   double* T;                   // [nz] zone temperature, replaced
   int32_t* n_unsolved;         // zones where Brent hit its iteration limit
 };
-// radiative-equilibrium temperature of every zone (one thread per zone)
-int launch_temperature(const TemperatureArgs& a, cudaStream_t s);
+// radiative-equilibrium temperature of every zone
+int launch_temperature(const TemperatureArgs& a, int num_sms, cudaStream_t s);
 
 // ---------------------------------------------------------------- opacity
 struct OpacityArgs {
