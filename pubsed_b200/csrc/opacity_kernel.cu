@@ -3,7 +3,7 @@
 //
 //   zone_state_warp_kernel
 //                       one warp per zone (zone_state_kernel, one thread,
-//                       for very long level lists): temperature clamp, mass
+//                       for very long level lists and many zones of short ones): temperature clamp, mass
 //                       fractions, then the LTE electron-density solve
 //                       (GasState::solve_state / ne_brent_method,
 //                       src/opacity/GasState.cpp:208-337) with
@@ -166,8 +166,8 @@ __device__ __forceinline__ double zone_mass_fractions(const OpacityArgs& A, int 
 }
 
 // One thread per zone: the form for level lists too long for the shared
-// memory of zone_state_warp_kernel, and for FP64 chunks of very many zones
-// (launch_zone_state).
+// memory of zone_state_warp_kernel, and for many zones of short ones
+// (zone_state_by_thread).
 __global__ void zone_state_kernel(const OpacityArgs A, double* boltz_e)
 {
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
@@ -379,17 +379,29 @@ __global__ void __launch_bounds__(32 * ZONE_WARPS) zone_state_warp_kernel(const 
 // it (about 3000 levels in FP64, 6000 with FP32 tables) take one thread per
 // zone.
 constexpr size_t ZONE_STATE_SMEM = 200 * 1024;
-// FP64 chunks of more zones than this take one thread per zone: with the chip
-// full of threads either way, the summing lanes' idle neighbours cost the warp
-// form more than the shared state saves it (906 levels: 64 000 zones 5.55
-// against 5.91 ms, 262 144 zones 22.2 against 18.2 ms).
-constexpr int ZONE_STATE_FP64_WARP_ZONES = 65536;
+// Many zones fill the chip with a thread each, and a warp's 32 lanes then cost
+// more than the shared state saves: with short level lists most of them have
+// nothing to do in an evaluation, and in FP64 the lanes that sum an atom's
+// levels leave the others idle.  sed_set_opacity on B200 (4 bins, so mostly this
+// solve) in ms, a warp / a thread per zone:
+//   levels (atoms)      11 (1)       102 (2)      156 (6)      906 (6)
+//   FP64   4 096 zones  0.15 / 0.16  0.17 / 0.43  0.18 / 0.86  0.54 / 3.21
+//         32 768        0.97 / 0.40  1.15 / 0.77  1.25 / 1.26  3.45 / 6.52
+//        110 592        3.24 / 1.18  3.90 / 2.16  4.32 / 3.71  11.6 / 13.6
+//        262 144        7.66 / 2.84  9.25 / 4.66  10.1 / 7.34  26.4 / 23.0
+//   FP32  32 768        0.53 / 0.39  0.61 / 0.75  0.65 / 1.25  1.30 / 6.48
+//        262 144        4.07 / 2.62  4.95 / 4.46  5.29 / 7.12  9.64 / 22.3
+bool zone_state_by_thread(bool fast, int nz, int n_lev, int num_sms)
+{
+  if (nz < 128 * num_sms) return false;
+  return fast ? n_lev <= 64 : nz >= (int64_t)210 * n_lev;
+}
 
-int launch_zone_state(const OpacityArgs& a, cudaStream_t s)
+int launch_zone_state(const OpacityArgs& a, int num_sms, cudaStream_t s)
 {
   const bool fast = a.precision != 0;
   const size_t smem = ZONE_WARPS * sizeof(double) * zone_state_doubles(fast, a.natoms, a.n_ions_total, a.n_lev_total);
-  if (smem > ZONE_STATE_SMEM || (!fast && a.nzones > ZONE_STATE_FP64_WARP_ZONES)) {
+  if (smem > ZONE_STATE_SMEM || zone_state_by_thread(fast, a.nzones, a.n_lev_total, num_sms)) {
     zone_state_kernel<<<(a.nzones + 127) / 128, 128, 0, s>>>(a, a.boltz);
     return 1;
   }
@@ -1178,7 +1190,7 @@ int launch_opacity(const OpacityArgs& a, int num_sms, cudaStream_t s)
 {
   const int nz = a.nzones;
   int n = 0;
-  if (launch_zone_state(a, s) < 0) return -1;
+  if (launch_zone_state(a, num_sms, s) < 0) return -1;
   ++n;
   const bool micro = a.natoms > 0;
   int r = 0;
@@ -1295,6 +1307,8 @@ extern "C" int sed_lte_electron_density_noalloc(int32_t n_zones, const double* r
   // the array keeps the previous call's contents; only the grey-opacity
   // column must start at zero (every other entry is written before it is read)
   if (cudaMemsetAsync(grey, 0, nz * sizeof(double), s) != cudaSuccess) return SED_ERR_CUDA;
-  if (launch_zone_state(A, s) < 0) return SED_ERR_CUDA;
+  int num_sms = 0;
+  if (cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return SED_ERR_CUDA;
+  if (launch_zone_state(A, num_sms, s) < 0) return SED_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SED_OK : SED_ERR_CUDA;
 }
