@@ -356,15 +356,17 @@ struct Stream<0> {
   }
 };
 
-// the state emit_mixed_kernel stored for core packet q
+// the state emit_mixed_kernel stored for core packet q (by ordinary loads: the
+// read-only path is for what no thread of the kernel writes, and the 3D kernel
+// leaves escaped packets in these slots)
 __device__ __forceinline__ void load_emitted(const StepArgs& A, Pkt& p, int64_t q)
 {
   const int64_t n = A.em_n;
   const double* s = A.em_state + q;
-  p.x[0] = __ldg(s); p.x[1] = __ldg(s + n); p.x[2] = __ldg(s + 2 * n);
-  p.D[0] = __ldg(s + 3 * n); p.D[1] = __ldg(s + 4 * n); p.D[2] = __ldg(s + 5 * n);
-  p.t = __ldg(s + 6 * n); p.e = __ldg(s + 7 * n); p.nu = __ldg(s + 8 * n);
-  p.ind = __ldg(A.em_ind + q);
+  p.x[0] = s[0]; p.x[1] = s[n]; p.x[2] = s[2 * n];
+  p.D[0] = s[3 * n]; p.D[1] = s[4 * n]; p.D[2] = s[5 * n];
+  p.t = s[6 * n]; p.e = s[7 * n]; p.nu = s[8 * n];
+  p.ind = A.em_ind[q];
 }
 
 }  // namespace mixed
