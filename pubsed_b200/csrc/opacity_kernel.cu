@@ -974,8 +974,9 @@ __global__ void __launch_bounds__(THREADS, BF ? 1 : 1024 / THREADS) zone_opacity
   // where a serial row per CTA would dominate the build) a blocked scan in a
   // fixed order: each warp scans a contiguous run of bins 32 at a time, the
   // run totals are added up in order, each run adds its offset; non-negative
-  // terms, so every prefix is within a few ulp of the sequential sum, and a
-  // NaN term propagates to the end as in the sequential sum.
+  // terms, so every prefix is within a few ulp of the sequential sum and none is
+  // below the one before it, and a NaN term propagates to the end as in the
+  // sequential sum.
   double* em = R2;
   double Lth = 0;
   if (nn == 1) {
@@ -1005,10 +1006,20 @@ __global__ void __launch_bounds__(THREADS, BF ? 1 : 1024 / THREADS) zone_opacity
       const int j = jb + lane;
       double v = (j < j1) ? em[j] * __ldg(tab + BT_D * nn + j) : 0.0;
       Lp += 4 * PI * v;
+      const bool rises = __all_sync(0xffffffffu, !(v < 0));
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const double u = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += u;
+      }
+      // two lanes' sums round on their own: where the terms are small the later
+      // one may come out an ulp below, so each takes the largest up to it
+      if (rises) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o && u > v) v = u;
+        }
       }
       v += base;
       if (j < j1) em[j] = v;
