@@ -278,8 +278,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_fp64_kernel(const Ste
     if (d_nu < d_bn) { d_bn = d_nu; new_ind = iz; }
     const double tot_lab = op * dshift;
     const double tau_r = -1.0 * log(1 - u_tau);
-    double d_sc = div_rn(tau_r, tot_lab);
-    if (tot_lab == 0) d_sc = INFINITY;
+    const double d_sc = flight(tau_r, tot_lab);
     double d_tm = (A.tstop - p.t) * C_LIGHT;
     if (A.steady) d_tm = INFINITY;
     int event;
@@ -321,7 +320,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_fp64_kernel(const Ste
       // transport::do_scatter (scatter.cpp:12-70): draws n .. n + 6 from the
       // depth's block and the three after it
       ++n_scat;
-      const double eps = (op == 0) ? 0 : div_rn(a_opac, op);
+      const double eps = absorbed_part(a_opac, op);
       const PhiloxOut o1 = rng.block(A, c0 + 1), o2 = rng.block(A, c0 + 2);
       const double z1 = odd ? u01(o1.w[0], o1.w[1]) : u01(o0.w[2], o0.w[3]);
       ++rng.n;

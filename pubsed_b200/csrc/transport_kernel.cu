@@ -174,6 +174,14 @@ __device__ __forceinline__ double absorbed_part(double a_opac, double op)
   if (op > 1e-290 && op < 1e290) return div_rn(a_opac, op);
   return (op == 0) ? 0 : a_opac / op;
 }
+// the flight to optical depth tau: endless without opacity, and of no length
+// through an infinite one, where div_rn has no residual
+__device__ __forceinline__ double flight(double tau, double opac)
+{
+  double d = div_rn(tau, opac);
+  if (opac == 0) d = INFINITY;
+  return isinf(opac) ? 0.0 : d;
+}
 
 // Fluid at rest (static grids): every Doppler factor is exactly 1, and a
 // transform leaves only the division of D by its square (relativity.cpp:120-126).
@@ -840,8 +848,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_kernel(const StepArgs
       if (d_nu < d_bn) { d_bn = d_nu; new_ind = p.ind; }
       const double tot_lab = (MODE == 0 ? op : s_opac) * dshift;
       const double tau_r = -1.0 * log(1 - rng.next());
-      double d_sc = div_rn(tau_r, tot_lab);
-      if (tot_lab == 0) d_sc = INFINITY;
+      const double d_sc = flight(tau_r, tot_lab);
       double d_tm = (A.tstop - p.t) * C_LIGHT;
       if (A.steady) d_tm = INFINITY;
       int event;
