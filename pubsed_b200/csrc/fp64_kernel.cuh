@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_fp64_kernel(const Ste
                 const int m = (lo + hi) >> 1;
                 if (__ldg(row + m) <= u_cdf) lo = m + 1; else hi = m;
               }
+              lo = min(lo, nn - 1);
             } else {
               lo = cdf_row_sample<double>(A, p.ind, u_cdf);
             }

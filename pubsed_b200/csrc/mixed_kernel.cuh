@@ -183,7 +183,6 @@ __device__ __forceinline__ SampledBin sample_bin(const StepArgs& A, int iz, doub
     return s;
   }
   s.k = cdf_row_sample<float>(A, iz, u);
-  if (s.k > nn - 1) s.k = nn - 1;
   const float* row = reinterpret_cast<const float*>(A.cdf) + (size_t)iz * nn;
   s.c0 = (s.k == 0) ? 0.f : __ldg(row + s.k - 1);
   s.c1 = __ldg(row + s.k);
@@ -273,8 +272,7 @@ __device__ __forceinline__ int scatter_batch(const StepArgs& A, Pkt& p, double r
     if (nn == 1) p.nu = loc_sample(A.nu, 0, 0.5);
     else {
       const double u = (double)w_cdf * (1.0 / 4294967296.0);
-      int k = cdf_row_sample<float>(A, p.ind, u);
-      if (k > nn - 1) k = nn - 1;
+      const int k = cdf_row_sample<float>(A, p.ind, u);
       const float* row = reinterpret_cast<const float*>(A.cdf) + (size_t)p.ind * nn;
       const double lo = (k == 0) ? 0.0 : (double)__ldg(row + k - 1);
       const double hi = (double)__ldg(row + k);

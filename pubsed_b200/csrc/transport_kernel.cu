@@ -309,22 +309,24 @@ struct GridZoneOf {
 };
 
 // upper_bound(CDF row of zone iz, u): through the guide table when there is
-// one, else the two-level search over the coarse table
+// one, else the two-level search over the coarse table; the last bin where a
+// loaded row ends at or below u
 template <typename CT>
 __device__ __forceinline__ int cdf_row_sample(const StepArgs& A, int iz, double u)
 {
   const int nn = A.nu.n;
   const CT* row = reinterpret_cast<const CT*>(A.cdf) + (size_t)iz * nn;
-  if (A.cdf_guide) return upper_bound_guided<CT>(row, A.cdf_guide + (size_t)iz * (A.guide_n + 1), A.guide_n, u);
+  if (A.cdf_guide)
+    return min(upper_bound_guided<CT>(row, A.cdf_guide + (size_t)iz * (A.guide_n + 1), A.guide_n, u), nn - 1);
   const CT* crow = reinterpret_cast<const CT*>(A.cdf_coarse) + (size_t)iz * A.n_coarse;
-  return upper_bound_2level<CT>(row, crow, nn, A.n_coarse, u);
+  return min(upper_bound_2level<CT>(row, crow, nn, A.n_coarse, u), nn - 1);
 }
 
 template <typename CT>
 __device__ __forceinline__ int cdf_sample(const CT* __restrict__ y, int n, double u)
 {
   if (n == 1) return 0;
-  return upper_bound_t<CT>(y, n, u);
+  return min(upper_bound_t<CT>(y, n, u), n - 1);
 }
 
 // transport::isotropic_scatter (src/transport/scatter.cpp:303-351)
