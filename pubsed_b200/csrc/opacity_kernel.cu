@@ -252,6 +252,8 @@ __global__ void __launch_bounds__(32 * ZONE_WARPS) zone_state_warp_kernel(const 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nz = A.nzones, na = A.natoms, nI = A.n_ions_total, nL = A.n_lev_total;
   const int z0 = blockIdx.x * ZONE_WARPS, z = z0 + warp;
+  // entries in use: a caller may give room for more than the lists hold
+  const int nIu = (na > 0) ? min(nI, A.ion_off[na]) : 0, nLu = (na > 0) ? min(nL, A.lev_off[na]) : 0;
   const size_t per = zone_state_doubles(FAST, na, nI, nL);
   double* lev = zsm + warp * per;           // [nL] Boltzmann factors, then the populations (FAST); else the
   double* eb = FAST ? lev : lev + nL;       // terms of the sums, then the populations, beside the factors
@@ -274,9 +276,9 @@ __global__ void __launch_bounds__(32 * ZONE_WARPS) zone_state_warp_kernel(const 
     if (micro) {
       __syncwarp();  // lane 0's mass fractions
       for (int a = lane; a < na; a += 32) nd[a] = dens * A.mass_frac[(size_t)a * nz + z] / (A.eA[a] * MASS_P);
-      for (int l = lane; l < nL; l += 32) eb[l] = exp(-A.lev_E[l] / K_EV / T);
+      for (int l = lane; l < nLu; l += 32) eb[l] = exp(-A.lev_E[l] / K_EV / T);
       __syncwarp();
-      for (int i = lane; i < nI; i += 32) {  // a stage's levels in order, a lane per stage
+      for (int i = lane; i < nIu; i += 32) {  // a stage's levels in order, a lane per stage
         int a = 0;
         while (A.ion_off[a + 1] <= i) ++a;
         const int ion = i - A.ion_off[a], l1 = A.lev_off[a + 1];
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(32 * ZONE_WARPS) zone_state_warp_kernel(const 
         part[i] = sum;
       }
       __syncwarp();
-      for (int i = lane; i < nI; i += 32) {
+      for (int i = lane; i < nIu; i += 32) {
         int a = 0;
         while (A.ion_off[a + 1] <= i) ++a;
         if (i > A.ion_off[a]) coef[i] = exp(-1.0 * A.ion_chi[i - 1] / K_EV / T) * (part[i] / part[i - 1]);
@@ -369,9 +371,9 @@ __global__ void __launch_bounds__(32 * ZONE_WARPS) zone_state_warp_kernel(const 
     }
   };
   const size_t o = (FAST ? 1 : 2) * (size_t)nL;
-  put(A.lev_n, 0, nL);
-  put(A.ion_part, o, nI);
-  put(A.ion_frac, o + nI, nI);
+  put(A.lev_n, 0, nLu);
+  put(A.ion_part, o, nIu);
+  put(A.ion_frac, o + nI, nIu);
   put(A.n_dens, o + 3 * (size_t)nI, na);
 }
 
