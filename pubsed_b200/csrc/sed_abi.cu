@@ -853,8 +853,7 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
       c->d_em_ind.release();
     }
   }
-  // (on a 3D grid of few cells too, where direct adds would meet on the same addresses)
-  if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G)) || (cart_path(A, G) && nz <= 8192)) {
+  if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G)) || (cart_path(A, G) && nz <= CART_COPY_ZONES)) {
     const int rc_rep = zone_tally_copies(c, A);
     if (rc_rep) return rc_rep;
   }

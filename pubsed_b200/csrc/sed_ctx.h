@@ -319,6 +319,10 @@ int enqueue_opacity(sed_ctx* c, double dt);
 // kernel arguments and device grid of a transport step of this context
 // the packed bins again, after the {abs, scat} or CDF tables were written by something else than an opacity build
 cudaError_t pack_bins(sed_ctx* c);
+// 3D grids of up to this many cells take the copies of the zone tallies below
+// where their kernel has FP32 tables: with few cells direct adds meet on the
+// same addresses
+constexpr size_t CART_COPY_ZONES = 8192;
 // the zone-scalar tallies of a step in copies (zeroed), for the packet and finish kernels
 int zone_tally_copies(sed_ctx* c, StepArgs& A);
 // the same for the mean intensity, where it is small

@@ -173,8 +173,8 @@ int diff_forward(sed_ctx* c, double dt, const double* abs_scale, cudaMemcpyKind 
     A.rec_fate = c->d_rec_fate.p; A.rec_ind = c->d_rec_ind.p; A.rec_draws = c->d_rec_draws.p; A.rec_state = c->d_rec_state.p;
   }
   const GridDev G = make_grid_dev(c);
-  if (c->gtype == SED_GRID_1D_SPHERE && c->tp.precision) {
-    // zone-scalar tallies in copies, as for the 1D packet kernels of a plain step
+  if (c->tp.precision && (c->gtype == SED_GRID_1D_SPHERE || nz <= CART_COPY_ZONES)) {
+    // zone-scalar tallies in copies, as for the packet kernels of a plain step
     const int rc_rep = zone_tally_copies(c, A);
     if (rc_rep) return rc_rep;
   }
