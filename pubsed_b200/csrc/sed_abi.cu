@@ -695,6 +695,21 @@ static int build_census(sed_ctx* c, CensusArgs& C, int64_t n_all, int64_t* n_ali
   return SED_OK;
 }
 
+// The 3D kernel does without the emission slots, so a step takes them only where
+// they leave half of the free memory to what comes after: 2e9 packets would take
+// 152 GB, and the next step's tables or another context would find none.
+static bool emit_ahead_fits(sed_ctx* c, int64_t n)
+{
+  const size_t need = (size_t)n * (9 * sizeof(double) + sizeof(int32_t));
+  if (c->d_em_state.cap >= (size_t)n * 9 && c->d_em_ind.cap >= (size_t)n) return true;
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return need <= free_bytes / 2;
+}
+
 static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms_opacity)
 {
   if (!c) return SED_ERR_ARG;
@@ -843,16 +858,6 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
     CK(c->d_em_tau.resize((size_t)n_emit));
     A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_tau = c->d_em_tau.p; A.em_n = n_emit;
   }
-  if (cart_path(A, G) && n_emit > 0 && n_q == 0) {
-    // core packets emitted ahead where the memory holds them (80 B each), in the packet kernel otherwise
-    if (c->d_em_state.resize((size_t)n_emit * 9) == cudaSuccess && c->d_em_ind.resize((size_t)n_emit) == cudaSuccess) {
-      A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_n = n_emit;
-    } else {
-      cudaGetLastError();
-      c->d_em_state.release();
-      c->d_em_ind.release();
-    }
-  }
   if (mixed_1d_path(A, G) || (G.type == 0 && fp64_path(A, G)) || (cart_path(A, G) && nz <= CART_COPY_ZONES)) {
     const int rc_rep = zone_tally_copies(c, A);
     if (rc_rep) return rc_rep;
@@ -860,6 +865,16 @@ static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms
   {
     const int rc_rep = J_tally_copies(c, A);
     if (rc_rep) return rc_rep;
+  }
+  if (cart_path(A, G) && n_emit > 0 && n_q == 0 && emit_ahead_fits(c, n_emit)) {
+    // core packets emitted ahead (76 B each) where the memory has the room, in the packet kernel otherwise
+    if (c->d_em_state.resize((size_t)n_emit * 9) == cudaSuccess && c->d_em_ind.resize((size_t)n_emit) == cudaSuccess) {
+      A.em_state = c->d_em_state.p; A.em_ind = c->d_em_ind.p; A.em_n = n_emit;
+    } else {
+      cudaGetLastError();
+      c->d_em_state.release();
+      c->d_em_ind.release();
+    }
   }
   CK(cudaEventRecord(c->ev[3], c->stream));
   if (A.n_packets > 0) launches += launch_propagate(A, G, c->num_sms, c->stream);
