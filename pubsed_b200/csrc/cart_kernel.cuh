@@ -17,17 +17,6 @@
 // ones binned into the spectrum afterwards, so neither long stretch holds a
 // warp for one of its lanes.
 
-// walls pushed across by 1e-10 of the cell, as get_next_zone
-// (grid_3D_cart.cpp:396-469) forms them: {left, right} per cell of an axis
-__global__ void pushed_walls_kernel(const DevLoc ax, double2* __restrict__ out)
-{
-  const double tiny = 1e-10;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ax.n; i += gridDim.x * blockDim.x) {
-    const double dd = loc_delta(ax, i);
-    out[i] = make_double2(loc_left(ax, i) - dd * tiny, __ldg(ax.right + i) + dd * tiny);
-  }
-}
-
 // EMIT = 0: a step of core packets alone, emitted ahead into em_state, where an
 // escaped packet's {t_obs, e, nu, D} are left for count_escaped_kernel (its
 // em_ind ESCAPED_SLOT); EMIT = 1: any step, packets emitted and counted here.

@@ -351,9 +351,17 @@ int sed_set_grid(sed_ctx* c, const sed_grid* g)
       c->ax[a] = host_loc(*axes[a]);
       CK(upload(c, c->d_ax[a], c->ax[a].x.data(), c->ax[a].x.size()));
     }
-    CK(c->d_ax_push.resize((size_t)c->nx + c->ny + c->nzz));
-    for (int a = 0, o = 0; a < 3; o += c->ax[a++].n()) launch_pushed_walls(dev_loc(c->ax[a], c->d_ax[a]), c->d_ax_push.p + o, c->stream);
-    CK(cudaGetLastError());
+    if (c->tp.precision) {
+      // walls pushed across by 1e-10 of the cell, as get_next_zone
+      // (grid_3D_cart.cpp:396-469) forms them, for the 3D mixed kernel: {left,
+      // right} per cell of the three axes, one after the other (formed on the
+      // device, by a launch per axis, they took 20 of an upload's 90 us)
+      std::vector<double2> push;
+      for (const HostLoc& ax : c->ax)
+        for (int i = 0; i < ax.n(); ++i)
+          push.push_back(make_double2(ax.left(i) - ax.delta(i) * 1e-10, ax.x[i] + ax.delta(i) * 1e-10));
+      CK(upload(c, c->d_ax_push, push.data(), push.size()));
+    }
   } else {
     return set_err(c, SED_ERR_ARG, "sed_set_grid: unknown grid type %d", g->type);
   }

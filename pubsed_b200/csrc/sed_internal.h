@@ -213,8 +213,6 @@ bool fp64_path(const StepArgs& a, const GridDev& g);
 // whether it runs the 3D mixed kernel (cart_kernel.cuh): with em_n core packets
 // emitted ahead when they are all the step has and the em_* buffers are given
 bool cart_path(const StepArgs& a, const GridDev& g);
-// the pushed walls of an axis for it
-int launch_pushed_walls(const DevLoc& ax, double2* out, cudaStream_t s);
 // IMD probabilities of the step (transport::compute_diffusion_probabilities)
 // from the zone Planck means into out[4][nz]
 int launch_ddmc_geometry(const GridDev& g, double* out, cudaStream_t s);

@@ -2171,12 +2171,6 @@ bool cart_path(const StepArgs& a, const GridDev& g)
   return a.precision != 0 && g.type == 1 && g.homologous && a.use_ddmc == 0;
 }
 
-int launch_pushed_walls(const DevLoc& ax, double2* out, cudaStream_t s)
-{
-  pushed_walls_kernel<<<(ax.n + 127) / 128, 128, 0, s>>>(ax, out);
-  return 1;
-}
-
 int launch_imd_probabilities(const GridDev& g, const double* planck, double dt, double* out, cudaStream_t s)
 {
   imd_probabilities_kernel<<<(g.nzones + 127) / 128, 128, 0, s>>>(g, planck, dt, out);
