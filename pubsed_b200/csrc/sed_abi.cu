@@ -23,7 +23,7 @@ using namespace sed;
 namespace {
 
 // The packed bins of the 1D mixed packet kernel, 16 B a bin, for grids up to
-// this size (a larger grid, or one the memory does not hold, goes without: the
+// this size (a larger grid, or one that leaves no spare_room, goes without: the
 // kernel then reads the separate tables), and its guide tables, which are made
 // up to GUIDE_FINE times as fine as the bins as long as they stay in a quarter
 // of the L2: a finer guide settles more deviates with its first entry.  Type Ia,
@@ -31,6 +31,19 @@ namespace {
 // packed with a guide entry per bin 85.6, 2: 81.9, 4: 79.9, 8: 78.5.
 constexpr size_t BIN4_MAX_BYTES = size_t(8) << 30;
 constexpr size_t GUIDE_FINE = 8, GUIDE_FINE_BYTES = size_t(32) << 20;
+
+// Buffers that only make a step faster are taken where they leave half of the
+// free memory to what comes after (other buffers of the step, the next step's
+// tables, another context): the work then still fits where it fits without them.
+bool spare_room(size_t bytes)
+{
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= free_bytes / 2;
+}
 
 int alloc_tallies(sed_ctx* c)
 {
@@ -47,7 +60,8 @@ int alloc_tallies(sed_ctx* c)
   // packed bins: one model's 1D grid with FP32 tables
   c->d_bin4.release();
   if (c->tp.precision && c->gtype == SED_GRID_1D_SPHERE && !c->in_batch && nn > 1 && nn <= 65535 &&
-      nz * nn * sizeof(float4) <= BIN4_MAX_BYTES && c->d_bin4.resize(nz * nn) != cudaSuccess)
+      nz * nn * sizeof(float4) <= BIN4_MAX_BYTES && spare_room(nz * nn * sizeof(float4)) &&
+      c->d_bin4.resize(nz * nn) != cudaSuccess)
     cudaGetLastError();
   // guide tables: G = a power of two >= n_nu (uint16 bin indices)
   c->guide_n = 0;
@@ -703,19 +717,11 @@ static int build_census(sed_ctx* c, CensusArgs& C, int64_t n_all, int64_t* n_ali
   return SED_OK;
 }
 
-// The 3D kernel does without the emission slots, so a step takes them only where
-// they leave half of the free memory to what comes after: 2e9 packets would take
-// 152 GB, and the next step's tables or another context would find none.
+// The 3D kernel does without the emission slots (2e9 packets would take 152 GB)
 static bool emit_ahead_fits(sed_ctx* c, int64_t n)
 {
-  const size_t need = (size_t)n * (9 * sizeof(double) + sizeof(int32_t));
   if (c->d_em_state.cap >= (size_t)n * 9 && c->d_em_ind.cap >= (size_t)n) return true;
-  size_t free_bytes = 0, total = 0;
-  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return need <= free_bytes / 2;
+  return spare_room((size_t)n * (9 * sizeof(double) + sizeof(int32_t)));
 }
 
 static int transport_impl(sed_ctx* c, double dt, sed_step_stats* stats, float ms_opacity)
