@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_cart_kernel(const Ste
       // transport::do_scatter (scatter.cpp:12-70)
       s_scat[tid] += 1;
       int redist = 0;
-      const double eps = absorbed_part(a_opac, op);
+      const double eps = absorbed_part_rn(a_opac, op);
       if (!(w01(blk.z) > eps)) {
         if ((w01(blk.w) > eps_imc) || A.radiative_eq) redist = 1;
         else fate = ABSORBED;

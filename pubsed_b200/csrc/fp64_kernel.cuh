@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_fp64_kernel(const Ste
       // transport::do_scatter (scatter.cpp:12-70): draws n .. n + 6 from the
       // depth's block and the three after it
       ++n_scat;
-      const double eps = absorbed_part(a_opac, op);
+      const double eps = absorbed_part_rn(a_opac, op);
       const PhiloxOut o1 = rng.block(A, c0 + 1), o2 = rng.block(A, c0 + 2);
       const double z1 = odd ? u01(o1.w[0], o1.w[1]) : u01(o0.w[2], o0.w[3]);
       ++rng.n;

@@ -178,9 +178,15 @@ __device__ __forceinline__ double absorbed_part(double a_opac, double op)
 // through an infinite one, where div_rn has no residual
 __device__ __forceinline__ double flight(double tau, double opac)
 {
-  double d = div_rn(tau, opac);
-  if (opac == 0) d = INFINITY;
-  return isinf(opac) ? 0.0 : d;
+  const bool none = opac == 0, all = isinf(opac);
+  const double d = div_rn(tau, opac), end = none ? (double)INFINITY : 0.0;
+  return (none || all) ? end : d;
+}
+// absorbed_part without a branch, for opacities in the normal range or infinite
+__device__ __forceinline__ double absorbed_part_rn(double a_opac, double op)
+{
+  const double d = div_rn(a_opac, op);
+  return (op == 0 || (isinf(op) && !isinf(a_opac))) ? 0.0 : d;
 }
 
 // Fluid at rest (static grids): every Doppler factor is exactly 1, and a
