@@ -109,15 +109,23 @@ inline float lookup_margin(const HostLoc& h)
   if (h.type == LOC_LOG) {
     if (!(h.min > 1e-37 && top < 1e37)) return 1.f;  // 1/min and x as floats
     const double inv_step = 1.0 / std::log2(1.0 + h.del);
-    for (int i = 0; i + 1 < n; ++i)
-      off = std::max(off, std::fabs(std::log2(h.x[i] / h.min) * inv_step - (i + 1)));
+    for (int i = 0; i + 1 < n; ++i) {
+      const double d = std::fabs(std::log2(h.x[i] / h.min) * inv_step - (i + 1));
+      if (!(d < 1)) return 1.f;  // also a wall that is no number
+      off = std::max(off, d);
+    }
     err += 0x1p-22 * (1.1 + std::max(1.0, std::log2(top / h.min))) * inv_step;
   } else {
-    for (int i = 0; i + 1 < n; ++i) off = std::max(off, std::fabs((h.x[i] - h.min) / h.del - (i + 1)));
+    if (!(top - h.min < 1e37 && h.del > 1e-37 && h.del < 1e37)) return 1.f;  // x - min and 1/del as floats
+    for (int i = 0; i + 1 < n; ++i) {
+      const double d = std::fabs((h.x[i] - h.min) / h.del - (i + 1));
+      if (!(d < 1)) return 1.f;
+      off = std::max(off, d);
+    }
     err += 0x1p-52 * (std::fabs(h.min) + std::fabs(top)) / h.del;
   }
   const double m = std::max({1.0 / 64, n * 0x1p-18, 2 * err}) + off;
-  return m < 1 ? (float)m : 1.f;  // also when a wall is no number
+  return m < 1 ? (float)m : 1.f;
 }
 
 inline HostLoc host_loc(const sed_locate_grid& g)

@@ -25,7 +25,8 @@ def test_lookup_gives_the_walls_bin(sed_lib, tmp_path):
     f.argtypes = [C.c_int, C.c_int, C.c_double, C.c_double, C.c_void_p, C.c_ulonglong, C.c_void_p]
     log = lambda ratio, n: log_grid(6e14, 6e14 * ratio, ratio ** (1.0 / n) - 1.0)
     grids = [log(100, 4096), log(1.02, 4096), log(1.01, 2000), log(1.005, 1000), log(1.0001, 300), log(1.5, 60000),
-             log(1e6, 37), lin_grid(1e14, 1e16, 2.4e12), lin_grid(1e15, 1.001e15, 1e9), lin_grid(1e15, 1.0000001e15, 1e6)]
+             log(1e6, 37), lin_grid(1e14, 1e16, 2.4e12), lin_grid(1e15, 1.001e15, 1e9), lin_grid(1e15, 1.0000001e15, 1e6),
+             lin_grid(1e30, 1e40, 1.1e38)]
     bent = log(100, 500)
     bent.right = bent.right.copy()
     bent.right[:-1] *= 1 + 0.002 * np.sin(np.arange(bent.n - 1))
