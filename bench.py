@@ -102,6 +102,26 @@ def captured_issue(workload: str, n_segments: int, kernel_ms: float, sm_mhz, n_s
     return None
 
 
+def roofline(alg_bytes: float, kernel_ms: float, kernel: str, bound: str, traffic) -> dict:
+    """The packet kernel's algorithmic bytes per launch over its time, beside
+    the measured copy bandwidth.  The bytes are served by L1 and L2 before
+    DRAM, so `frac` is no bound the kernel meets; `dram_frac` is the captured
+    DRAM traffic over the same time and peak, and `bound` names what the
+    kernel waits for."""
+    peaks = {}
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            peaks = json.load(f)
+    except Exception:
+        pass
+    peak = float(peaks.get("hbm_gbs", 6650.0))
+    gbs = 1.0 / (kernel_ms * 1e-3) / 1e9
+    return {"bound": bound, "achieved": alg_bytes * gbs, "peak": peak, "unit": "GB/s", "frac": alg_bytes * gbs / peak,
+            "basis": "algorithmic bytes, served by L1, L2 and DRAM, against the HBM copy rate",
+            "traffic": traffic, "dram_frac": traffic * gbs / peak if traffic else None, "kernel": kernel,
+            "kernel_ms": kernel_ms, "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}
+
+
 def _env_rank():
     return int(os.environ.get("RANK", "0")), int(os.environ.get("WORLD_SIZE", "1")), int(os.environ.get("LOCAL_RANK", "0"))
 
@@ -411,18 +431,8 @@ def main_batch(args, rank: int, world: int, local: int):
         out["batched_fp64"] = {"value": n_total / (m64 * 1e-3), "ms_per_step": m64}
         b64.close()
     b_seg, b_pkt = 16 + 8 + 16 + 16 + 64, 264
-    achieved = (last["n_segments"] * b_seg + n_total * b_pkt) / (kern_ms * 1e-3) / 1e9
-    peaks = {}
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peaks = json.load(f)
-    except Exception:
-        pass
-    peak = float(peaks.get("hbm_gbs", 6650.0))
-    out["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                       "traffic": captured_traffic(bw.name, last["n_segments"]),
-                       "kernel": "propagate_mixed_kernel (batched)", "kernel_ms": kern_ms,
-                       "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}
+    out["roofline"] = roofline(last["n_segments"] * b_seg + n_total * b_pkt, kern_ms, "propagate_mixed_kernel (batched)",
+                               "issue", captured_traffic(bw.name, last["n_segments"]))
     out["clocks"] = clk.summary()
     out["roofline"]["issue"] = captured_issue(bw.name, last["n_segments"], kern_ms, out["clocks"].get("sm_mhz"),
                                               torch.cuda.get_device_properties(local).multi_processor_count)
@@ -525,14 +535,7 @@ def main_adjoint(args, rank: int, world: int, local: int):
               "norm": "||fd - adjoint||_2 / ||adjoint||_2 over the 1024 spectrum bins of a (zone, band) column"}
     value = n / ((ms_f + ms_b) * 1e-3)
     b_seg, b_pkt = 16 + 8 + 16 + 16 + 64, 264
-    achieved = (seg * b_seg + n * b_pkt) / (ms_k * 1e-3) / 1e9
-    peaks = {}
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peaks = json.load(f)
-    except Exception:
-        pass
-    peak = float(peaks.get("hbm_gbs", 6650.0))
+    alg_bytes = seg * b_seg + n * b_pkt
     out = {"metric": METRIC + " (forward + adjoint)", "value": value, "unit": UNIT, "n_gpus": world,
            "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_f + ms_b, "higher_is_better": True,
            "scaling": "weak", "vs_baseline": None, "dtype": "f64 transport / f32 opacity tables",
@@ -542,9 +545,7 @@ def main_adjoint(args, rank: int, world: int, local: int):
            "gpu_launches": 3 * args.steps,
            "e2e": {"value": n / e2e, "unit": UNIT, "h2d_bytes_per_step": int(theta.nbytes + g.nbytes),
                    "d2h_bytes_per_step": int(flux.nbytes + click.nbytes + grad.nbytes), "ms_per_step": e2e * 1e3},
-           "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                        "traffic": None, "kernel": "propagate_diff_kernel (weighted forward)", "kernel_ms": ms_k,
-                        "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},
+           "roofline": roofline(alg_bytes, ms_k, "propagate_diff_kernel (weighted forward)", "latency", None),
            "clocks": clk.summary()}
     if not args.no_cpu_baseline:
         out["cpu_baseline"] = ref.get("cpu_baseline", {"value": None, "sample": ref.get("unavailable")})
@@ -804,14 +805,6 @@ def main():
     b_seg = (24 if w.zones.type == abi.GRID_3D_CART else 16) + 8 + 16 + 16 + 64
     b_pkt = 264
     alg_bytes = last["n_segments"] * b_seg + args.packets * b_pkt
-    achieved = alg_bytes / (kern_ms * 1e-3) / 1e9
-    peaks = {}
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peaks = json.load(f)
-    except Exception:
-        pass
-    peak = float(peaks.get("hbm_gbs", 6650.0))
     traffic = captured_traffic(w.name, last["n_segments"], n_step)
 
     line = {
@@ -831,16 +824,13 @@ def main():
         "gpu_launches": int(sum(s["kernel_launches"] for s in stats)),
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                 "ms_per_step": e2e_t * 1e3},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": traffic,
-                     "kernel": "propagate_mixed_kernel" if w.zones.type != abi.GRID_3D_CART else "propagate_cart_kernel",
-                     "kernel_ms": kern_ms,
-                     "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},
+        "roofline": (roofline(alg_bytes, kern_ms, "propagate_cart_kernel", "DRAM latency", traffic)
+                     if w.zones.type == abi.GRID_3D_CART else
+                     roofline(alg_bytes, kern_ms, "propagate_mixed_kernel", "issue", traffic)),
         "clocks": clk.summary(),
     }
-    # what bounds the kernel: its tables stay in L2, so the HBM fraction
-    # above is nominal; the issue rate against the scheduler ceiling is the
-    # figure that moves with it
+    # the issue rate against the scheduler ceiling: what the 1D kernel, whose
+    # tables stay in L2, is bound by
     line["roofline"]["issue"] = captured_issue(w.name, last["n_segments"], kern_ms, line["clocks"].get("sm_mhz"),
                                                torch.cuda.get_device_properties(local).multi_processor_count)
     if radio_frac > 0:

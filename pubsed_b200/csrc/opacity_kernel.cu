@@ -863,9 +863,10 @@ __device__ __forceinline__ double warp_sum_f64(double v)
 // What bounds it: FP64 arithmetic per bin, then the serial parts of a row.
 // The bin constants come from bin_table_kernel, the sums and the scan are
 // warp shuffles, and the guide table is written bin by bin (below): 64^3 zones
-// x 2048 bins, FP32 tables, 31.7 -> 10.4 ms (its traffic, 11.8 GB, is 1.8 ms
-// of HBM), 18 494 zones 3.07 -> 0.94 ms, with bound-free levels (128 zones x
-// 2048 bins x 606 levels) 1.10 -> 0.48 ms.
+// x 2048 bins, FP32 tables, 31.7 -> 11.6 ms (1.2 of it so that no sum of the
+// scan falls; its traffic, 11.8 GB, is 1.8 ms of HBM), 18 494 zones 3.07 -> 1.02
+// ms, with bound-free levels (128 zones x 2048 bins x 606 levels) 1.10 -> 0.48
+// ms.
 template <bool MIXED, int THREADS, bool BF>
 __global__ void __launch_bounds__(THREADS, BF ? 1 : 1024 / THREADS) zone_opacity_kernel(const OpacityArgs A)
 {

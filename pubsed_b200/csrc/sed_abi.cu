@@ -192,9 +192,12 @@ int sed::zone_tally_copies(sed_ctx* c, StepArgs& A)
 // frequency bin (grey transport), or J not stored per bin.  The L2 takes the
 // adds of one address one after the other, so blocks spread over copies: the
 // diffusing pulse's packet kernel (200 zones, one bin, 1e6 packets, 41e6 adds)
-// ran 17.9 ms on one tally, 7.2 ms on 4 copies and on 32.  From 1e5 bins on
-// (97 zones x 1500, 128 x 1024) copies changed nothing, so they end at
-// J_COPIES_SIZE doubles.
+// ran 17.9 ms on one tally, 7.2 ms on 4 copies and on 32.  Grey sphere, 3e5
+// packets, packet kernel on 1 / 2 / 8 / 32 copies: 100 values FP64 27.4 / 17.8 /
+// 7.2 / 6.9 ms, mixed 28.0 / 18.6 / 6.7 / 4.3; 1024 values 10.9 / 10.4 / 10.2 / 10.3
+// and 11.1 / 8.0 / 6.3 / 6.2; 4096 values 9.5 / 9.7 / 9.6 / 9.6 and 7.4 / 6.2 / 6.3 /
+// 6.4; from 8192 values on within the spread, so two copies or more are taken as
+// long as all of them stay within J_COPIES_SIZE doubles: up to 32768 values.
 int sed::J_tally_copies(sed_ctx* c, StepArgs& A)
 {
   constexpr size_t J_COPIES_SIZE = size_t(1) << 16;

@@ -213,9 +213,10 @@ bool fp64_path(const StepArgs& a, const GridDev& g);
 // whether it runs the 3D mixed kernel (cart_kernel.cuh): with em_n core packets
 // emitted ahead when they are all the step has and the em_* buffers are given
 bool cart_path(const StepArgs& a, const GridDev& g);
+// the wall factors of the DDMC leakage opacities into out[3][nz]
+int launch_ddmc_geometry(const GridDev& g, double* out, cudaStream_t s);
 // IMD probabilities of the step (transport::compute_diffusion_probabilities)
 // from the zone Planck means into out[4][nz]
-int launch_ddmc_geometry(const GridDev& g, double* out, cudaStream_t s);
 int launch_imd_probabilities(const GridDev& g, const double* planck, double dt, double* out, cudaStream_t s);
 // zone-scalar tally normalisation (reduce_radiation) and steady-state rescale
 int launch_finish(const StepArgs& a, const GridDev& g, const double* vol, int64_t nspec, cudaStream_t s);

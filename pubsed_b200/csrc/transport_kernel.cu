@@ -2093,10 +2093,13 @@ int launch_propagate_t(const StepArgs& a, const GridDev& g, int num_sms, cudaStr
     else return launch_cart(a, g, num_sms, s);
   } else {
     if (fp64_ok(a, g)) {
-      // few packets wait for the longest chain: 16 warps per SM at 112
+      // few packets wait for the longest chain: 16 warps per SM at 114
       // registers; many fill the SM: 24 warps at 80 (Type Ia, packet kernel:
-      // 3e5 packets 92 against 108 ms, 1e6 151 against 158, 2e6 274 against
-      // 241 ms; grey lightbulb 1e5 6.5 against 7.1, 1e6 31.0 against 28.0 ms)
+      // 3e5 packets 94 against 112 ms, 6e5 119 against 120, 1e6 161 against
+      // 160, 2e6 273 against 251 ms; grey lightbulb 1e5 6.5 against 7.1, 1e6
+      // 31.0 against 28.0 ms).  3D grids take the same line, though their
+      // chains are shorter: 64^3 cells, 5e4 packets 6.0 against 6.5, 3e5 13.5
+      // against 12.9, 6e5 22.7 against 21.1, 1e6 35.5 against 32.1 ms.
       if (a.n_packets < (int64_t)num_sms * 768 * 8) return launch_fp64_t<GRID, 0, 128, 4>(a, g, 0, num_sms, a.n_packets, s);
       return launch_fp64_t<GRID, 0, 256, 3>(a, g, 0, num_sms, a.n_packets, s);
     }
