@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_cart_kernel(const Ste
         else fate = ABSORBED;
       }
       if (fate == MOVING) {
-        isotropic_scatter_fast<float>(A, p, philox_words(A, stream, n_blk), redist);
+        isotropic_scatter_fast(A, p, philox_words(A, stream, n_blk), redist);
         ++n_blk;
         directions();
       }

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, MINB) propagate_diff_kernel(const Ste
       }
     } else if (event == 0) {
       ++n_scat;
-      isotropic_scatter_fast<float>(A, p, block(n_blk), 0);
+      isotropic_scatter_fast(A, p, block(n_blk), 0);
       ++n_blk;
     } else {
       fate = STOPPED;

@@ -393,7 +393,6 @@ __device__ __forceinline__ double dshift_fast(const StepArgs& A, double rsq, dou
 // transport::isotropic_scatter (scatter.cpp:303-351), homologous flow
 // Its deviates are the four words of one Philox block: mu, phi, the
 // emissivity-CDF deviate and the position within the bin.
-template <typename CT>
 __device__ __forceinline__ void isotropic_scatter_fast(const StepArgs& A, Pkt& p, const uint4 w, int redist)
 {
   const double b0 = p.x[0] * A.inv_ct, b1 = p.x[1] * A.inv_ct, b2 = p.x[2] * A.inv_ct;  // v / c
@@ -417,7 +416,7 @@ __device__ __forceinline__ void isotropic_scatter_fast(const StepArgs& A, Pkt& p
   if (redist) {  // transport::sample_photon_frequency (emission.cpp:27-46)
     const int nn = A.nu.n;
     const double u = w01(w.z);
-    const int inu = (nn == 1) ? 0 : cdf_row_sample<CT>(A, p.ind, u);
+    const int inu = (nn == 1) ? 0 : cdf_row_sample<float>(A, p.ind, u);
     p.nu = loc_sample(A.nu, inu, w01(w.w));
   }
   // comoving -> lab with the velocity reversed: beta' = -beta
